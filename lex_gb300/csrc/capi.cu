@@ -582,9 +582,16 @@ int lexgb_destroy(lexgb_ctx* c) {
 
 int lexgb_set_stream(lexgb_ctx* c, void* stream) {
   if (!c) return fail(LEXGB_ERR_ARG, "null context");
+  // Binding the stream that is bound already changes nothing: the work stays in its order and the
+  // step graph stays.  autograd.set_state / get_state bind torch's current stream on every call;
+  // synchronising and capturing the step again there cost about 300 us a call (16x16x12, one step
+  // between set_state and get_state: 520 us, of which the step itself 200).
+  const cudaStream_t next = stream ? (cudaStream_t)stream : c->own_stream;
+  if (next == c->stream) return LEXGB_OK;
+  // the graph is captured on the context's own stream and launched on the bound one, so it outlives
+  // a change of stream; the synchronisation keeps two replays from running at once
   CK(cudaStreamSynchronize(c->stream));
-  c->stream = stream ? (cudaStream_t)stream : c->own_stream;
-  drop_graph(c);
+  c->stream = next;
   return LEXGB_OK;
 }
 

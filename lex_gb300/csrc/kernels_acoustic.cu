@@ -6,8 +6,8 @@
 //   pi'   <- pi' + 1.1 dtau (-(Rd/Cv)(pi0 + pi'_s) div(u) + adv_pi)
 //                                                 get_divergence2 / advection_pi, advection.py:152-236
 //
-// One thread per cell computes the new pi' of its cell and the new winds on the cell's west,
-// south and bottom faces; the winds on the east, north and top faces that its divergence needs
+// A thread computes the new pi' of its cells and the new winds on the cells' west, south and
+// bottom faces; the winds on the east, north and top faces that its divergence needs
 // are recomputed from the same inputs, so one launch is one whole sub-step.  Inputs and outputs
 // are distinct buffers (the caller ping-pongs).
 #include "lexgb_internal.cuh"
@@ -19,47 +19,12 @@ namespace {
 constexpr int BX = 32, BY = 4, BZ = 2;
 #define LD(p, idx) __ldg((p) + (idx))
 
-// x points per thread of the vectorised sub-step kernel
-#ifndef ACOUSTIC_VEC
-#define ACOUSTIC_VEC 4
-#endif
-// levels per thread of the vertical-march sub-step kernel (0: one level per thread)
-#ifndef ACOUSTIC_ZMARCH
-#define ACOUSTIC_ZMARCH 0
-#endif
-
 constexpr float kHalfCp = (float)(0.5 * kCp);
 constexpr float kRdCv = (float)(kRd / kCv);
 
 // -Cp * 0.5*(trho_a + trho_b) * ((p_a - p_b) * rd)
 __device__ __forceinline__ float pgf(float tra, float trb, float pa, float pb, float rd) {
   return -kHalfCp * (tra + trb) * ((pa - pb) * rd);
-}
-
-// new u on the west face of cell (i, j, k), i.e. u(i)
-__device__ __forceinline__ float u_new(const Dims& d, const Phys& ph, const AcousticIn& a, int i, int j, int k,
-                                       float dtau) {
-  const int im = wrap(i - 1, d.nx);
-  const int c0 = d.at(i, j, k), cm = d.at(im, j, k);
-  const float f = pgf(LD(a.trho, c0), LD(a.trho, cm), LD(a.p, c0), LD(a.p, cm), ph.rdx);
-  return LD(a.u, c0) + (f + LD(a.Ru, c0)) * dtau;
-}
-
-__device__ __forceinline__ float v_new(const Dims& d, const Phys& ph, const AcousticIn& a, int i, int j, int k,
-                                       float dtau) {
-  const int jm = wrap(j - 1, d.ny);
-  const int c0 = d.at(i, j, k), cm = d.at(i, jm, k);
-  const float f = pgf(LD(a.trho, c0), LD(a.trho, cm), LD(a.p, c0), LD(a.p, cm), ph.rdy);
-  return LD(a.v, c0) + (f + LD(a.Rv, c0)) * dtau;
-}
-
-// new w on face f (0..nz); zero on the bottom and the lid
-__device__ __forceinline__ float w_new(const Dims& d, const Phys& ph, const AcousticIn& a, int i, int j, int f,
-                                       float dtau) {
-  if (f <= 0 || f >= d.nz) return 0.f;
-  const int c0 = d.at(i, j, f), cm = d.at(i, j, f - 1);
-  const float g = pgf(LD(a.trho, c0), LD(a.trho, cm), LD(a.p, c0), LD(a.p, cm), ph.rdz);
-  return LD(a.w, c0) + (g + LD(a.Rw, c0)) * dtau;
 }
 
 // advection_pi at cell (i, j, k) given the face winds around it and pi'_s (advection.py:152-197)
@@ -80,30 +45,8 @@ __device__ __forceinline__ float adv_pi(const Dims& d, const Phys& ph, const Col
            (0.5f * wzb * c.rho_face[k] + 0.5f * wzt * c.rho_face[k + 1]) * c.rho_inv[k]);
 }
 
-__global__ void __launch_bounds__(BX* BY* BZ) k_acoustic(Dims d, Phys ph, Cols c, AcousticIn a, AcousticOut o,
-                                                       float dtau) {
-  const int i = blockIdx.x * BX + threadIdx.x, j = blockIdx.y * BY + threadIdx.y, k = blockIdx.z * BZ + threadIdx.z;
-  if (i >= d.nx || j >= d.ny || k >= d.nz) return;
-  const int ip = wrap(i + 1, d.nx), jp = wrap(j + 1, d.ny);
-  const float uw = u_new(d, ph, a, i, j, k, dtau);
-  const float ue = u_new(d, ph, a, ip, j, k, dtau);
-  const float vs = v_new(d, ph, a, i, j, k, dtau);
-  const float vn = v_new(d, ph, a, i, jp, k, dtau);
-  const float wb = w_new(d, ph, a, i, j, k, dtau);
-  const float wt = w_new(d, ph, a, i, j, k + 1, dtau);
-  const float div = (ue - uw) * ph.rdx + (vn - vs) * ph.rdy + (wt - wb) * ph.rdz;
-  const int id = d.at(i, j, k);
-  const float ap = adv_pi(d, ph, c, a.ps, i, j, k, uw, ue, vs, vn, wb, wt);
-  const float dpdt = -kRdCv * ((c.pi0[k] + LD(a.ps, id)) * div) + ap;
-  o.p[id] = LD(a.p, id) + (kDivDamp * dpdt) * dtau;
-  o.u[id] = uw;
-  o.v[id] = vs;
-  o.w[id] = wb;
-  if (k == d.nz - 1) o.w[d.at(i, j, d.nz)] = 0.f;
-}
-
-// Vectorised sub-step: each thread owns V (4 or 2) consecutive x points of one (j, k) row and
-// moves every field with V-wide loads/stores (needs nx % V == 0).  Same arithmetic as k_acoustic.
+// Each thread owns V (4, 2 or 1) consecutive x points of one (j, k) row and moves every field with
+// V-wide loads/stores (needs nx % V == 0).
 template <int V>
 struct VecT;
 template <>
@@ -113,6 +56,10 @@ struct VecT<4> {
 template <>
 struct VecT<2> {
   typedef float2 T;
+};
+template <>
+struct VecT<1> {
+  typedef float T;
 };
 
 template <int V>
@@ -141,16 +88,22 @@ __device__ __forceinline__ void zero(float (&o)[V]) {
 }
 
 template <int V>
-__global__ void __launch_bounds__(256) k_acoustic_vec(Dims d, Phys ph, Cols c, AcousticIn a, AcousticOut o,
-                                                      float dtau, int rev) {
+__global__ void __launch_bounds__(V == 4 ? 64 : 128, V == 4 ? 8 : 6) k_acoustic_vec(Dims d, Phys ph, Cols c, AcousticIn a, AcousticOut o,
+                                                      float dtau, int rev, int flat, int k0) {
+  pdl_wait();
+  pdl_trigger();
   const int nq = d.nx / V;
   // rev: blocks walk the grid in reverse order, so that a sub-step following one in forward order
   // starts on the fields its predecessor wrote last (still in L2)
   const int bx = rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
   const int by = rev ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
-  const int q = bx * blockDim.x + threadIdx.x;
-  const int j = by * blockDim.y + threadIdx.y;
-  const int k = rev ? gridDim.z - 1 - blockIdx.z : blockIdx.z;
+  int q = bx * blockDim.x + threadIdx.x;
+  int j = by * blockDim.y + threadIdx.y;
+  const int k = k0 + (rev ? gridDim.z - 1 - blockIdx.z : blockIdx.z);
+  if (flat) {   // consecutive points of the level, rows run together
+    j = q / nq;
+    q -= j * nq;
+  }
   if (q >= nq || j >= d.ny) return;
   const int nx = d.nx, nz = d.nz;
   const int i0 = q * V;
@@ -260,137 +213,6 @@ __global__ void __launch_bounds__(256) k_acoustic_vec(Dims d, Phys ph, Cols c, A
     float z[V];
     zero<V>(z);
     stv<V>(o.w, rt + i0, z);
-  }
-}
-
-// Vertical-march sub-step: each thread owns V consecutive x points of row j and walks the levels
-// kb .. kb+kc-1.  pi', theta_rho and pi'_s of the level above and the new w on the top face are
-// carried to the next level (the new w on face k+1 is the next level's bottom wind, same
-// operands), so each level loads 17 vectors instead of 25.  Same arithmetic as k_acoustic_vec.
-template <int V>
-__global__ void __launch_bounds__(256) k_acoustic_zm(Dims d, Phys ph, Cols c, AcousticIn a, AcousticOut o,
-                                                     float dtau, int kc) {
-  const int nq = d.nx / V;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (q >= nq || j >= d.ny) return;
-  const int nx = d.nx, nz = d.nz, plane = d.plane();
-  const int kb = blockIdx.z * kc, ke = min(kb + kc, nz);
-  const int i0 = q * V;
-  const int iw = wrap(i0 - 1, nx), ie = wrap(i0 + V, nx);
-  const int rc = j * nx, rs = wrap(j - 1, d.ny) * nx, rn = wrap(j + 1, d.ny) * nx;
-  float P[V], TR[V], S0[V], PB[V], TB[V], SB[V], WB[V];
-  ldv<V>(a.p, kb * plane + rc + i0, P);
-  ldv<V>(a.trho, kb * plane + rc + i0, TR);
-  ldv<V>(a.ps, kb * plane + rc + i0, S0);
-  if (kb > 0) {
-    const int rb = (kb - 1) * plane + rc + i0;
-    float W[V], RW[V];
-    ldv<V>(a.p, rb, PB);
-    ldv<V>(a.trho, rb, TB);
-    ldv<V>(a.ps, rb, SB);
-    ldv<V>(a.w, kb * plane + rc + i0, W);
-    ldv<V>(a.Rw, kb * plane + rc + i0, RW);
-#pragma unroll
-    for (int l = 0; l < V; ++l) WB[l] = W[l] + (pgf(TR[l], TB[l], P[l], PB[l], ph.rdz) + RW[l]) * dtau;
-  } else {
-    zero<V>(PB); zero<V>(TB); zero<V>(SB); zero<V>(WB);
-  }
-  for (int k = kb; k < ke; ++k) {
-    const int r0 = k * plane;
-    const bool has_b = k > 0, has_t = k + 1 < nz;
-    float U[V], RU[V], Vv[V], RV[V], VN[V], RVN[V], PS[V], TS[V], SS[V], PN[V], TN[V], SN[V];
-    float PT[V], TT[V], ST[V], WT[V], RWT[V];
-    ldv<V>(a.u, r0 + rc + i0, U);
-    ldv<V>(a.Ru, r0 + rc + i0, RU);
-    ldv<V>(a.v, r0 + rc + i0, Vv);
-    ldv<V>(a.Rv, r0 + rc + i0, RV);
-    ldv<V>(a.v, r0 + rn + i0, VN);
-    ldv<V>(a.Rv, r0 + rn + i0, RVN);
-    ldv<V>(a.p, r0 + rs + i0, PS);
-    ldv<V>(a.trho, r0 + rs + i0, TS);
-    ldv<V>(a.ps, r0 + rs + i0, SS);
-    ldv<V>(a.p, r0 + rn + i0, PN);
-    ldv<V>(a.trho, r0 + rn + i0, TN);
-    ldv<V>(a.ps, r0 + rn + i0, SN);
-    const float pW = __ldg(a.p + r0 + rc + iw), pE = __ldg(a.p + r0 + rc + ie);
-    const float tW = __ldg(a.trho + r0 + rc + iw), tE = __ldg(a.trho + r0 + rc + ie);
-    const float uE = __ldg(a.u + r0 + rc + ie), ruE = __ldg(a.Ru + r0 + rc + ie);
-    const float sW = __ldg(a.ps + r0 + rc + iw), sE = __ldg(a.ps + r0 + rc + ie);
-    if (has_t) {
-      const int rt = r0 + plane + rc + i0;
-      ldv<V>(a.p, rt, PT);
-      ldv<V>(a.trho, rt, TT);
-      ldv<V>(a.ps, rt, ST);
-      ldv<V>(a.w, rt, WT);
-      ldv<V>(a.Rw, rt, RWT);
-    } else {
-      zero<V>(PT); zero<V>(TT); zero<V>(ST); zero<V>(WT); zero<V>(RWT);
-    }
-    float un[V + 1];
-    {
-      float pc[V + 2], tc[V + 2], uc[V + 1], rcu[V + 1];
-      pc[0] = pW;
-      tc[0] = tW;
-      pc[V + 1] = pE;
-      tc[V + 1] = tE;
-      uc[V] = uE;
-      rcu[V] = ruE;
-#pragma unroll
-      for (int l = 0; l < V; ++l) {
-        pc[l + 1] = P[l];
-        tc[l + 1] = TR[l];
-        uc[l] = U[l];
-        rcu[l] = RU[l];
-      }
-#pragma unroll
-      for (int l = 0; l <= V; ++l) un[l] = uc[l] + (pgf(tc[l + 1], tc[l], pc[l + 1], pc[l], ph.rdx) + rcu[l]) * dtau;
-    }
-    float sc[V + 2];
-    sc[0] = sW;
-    sc[V + 1] = sE;
-#pragma unroll
-    for (int l = 0; l < V; ++l) sc[l + 1] = S0[l];
-    const float rho = c.rho[k], rhoi = c.rho_inv[k], rfb = c.rho_face[k], rft = c.rho_face[k + 1];
-    const float dzb = c.dpi0dz[k], dzt = c.dpi0dz[k + 1], pi0 = c.pi0[k];
-    float outp[V], outv[V], wt[V];
-#pragma unroll
-    for (int l = 0; l < V; ++l) {
-      const float p0 = P[l], t0 = TR[l];
-      const float vs = Vv[l] + (pgf(t0, TS[l], p0, PS[l], ph.rdy) + RV[l]) * dtau;
-      const float vn = VN[l] + (pgf(TN[l], t0, PN[l], p0, ph.rdy) + RVN[l]) * dtau;
-      const float wb = WB[l];
-      wt[l] = has_t ? WT[l] + (pgf(TT[l], t0, PT[l], p0, ph.rdz) + RWT[l]) * dtau : 0.f;
-      const float div = (un[l + 1] - un[l]) * ph.rdx + (vn - vs) * ph.rdy + (wt[l] - wb) * ph.rdz;
-      const float s0 = sc[l + 1];
-      const float gxw = (s0 - sc[l]) * ph.rdx, gxe = (sc[l + 2] - s0) * ph.rdx;
-      const float gys = (s0 - SS[l]) * ph.rdy, gyn = (SN[l] - s0) * ph.rdy;
-      const float wzb = has_b ? wb * (dzb + (s0 - SB[l]) * ph.rdz) : 0.f;
-      const float wzt = has_t ? wt[l] * (dzt + (ST[l] - s0) * ph.rdz) : 0.f;
-      const float ap = -(0.5f * (un[l + 1] * gxe + un[l] * gxw) + 0.5f * (vn * gyn + vs * gys) +
-                         (0.5f * wzb * rfb + 0.5f * wzt * rft) * rhoi);
-      const float dpdt = -kRdCv * ((pi0 + s0) * div) + ap;
-      outp[l] = p0 + (kDivDamp * dpdt) * dtau;
-      outv[l] = vs;
-    }
-    float outu[V];
-#pragma unroll
-    for (int l = 0; l < V; ++l) outu[l] = un[l];
-    stv<V>(o.p, r0 + rc + i0, outp);
-    stv<V>(o.u, r0 + rc + i0, outu);
-    stv<V>(o.v, r0 + rc + i0, outv);
-    stv<V>(o.w, r0 + rc + i0, WB);
-    if (k == nz - 1) {
-      float z[V];
-      zero<V>(z);
-      stv<V>(o.w, r0 + plane + rc + i0, z);
-    }
-#pragma unroll
-    for (int l = 0; l < V; ++l) {
-      PB[l] = P[l]; TB[l] = TR[l]; SB[l] = S0[l];
-      P[l] = PT[l]; TR[l] = TT[l]; S0[l] = ST[l];
-      WB[l] = wt[l];
-    }
   }
 }
 
@@ -745,40 +567,43 @@ __global__ void k_diag_advpi(Dims d, Phys ph, Cols c, const float* __restrict__ 
 
 }  // namespace
 
+template <int V>
+static cudaError_t launch_vec(const Dims& d, const Phys& ph, const Cols& c, const AcousticIn& in,
+                              const AcousticOut& out, float dtau, cudaStream_t st, int rev,
+                              const cudaAccessPolicyWindow* win) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[2] = {pdl_attribute()};
+  if (win) at[1] = window_attribute(*win);
+  cfg.attrs = at;
+  cfg.numAttrs = win ? 2 : 1;
+  cfg.stream = st;
+  // Blocks of 16 x 4 float4 (two warps, 8 blocks per SM: 128x128x64 8.5 us a sub-step with 16 x 16,
+  // 8.0 with 16 x 4; 32^3 2.24 and 2.03) where they fill the rows; else a block takes consecutive
+  // points of a level, rows run together, so that no lane is idle (102x75x59 6.1 -> 5.2 us, 240x240x120
+  // 57.5 -> 55.4; where the rows are filled the tile's y neighbours make it the faster one, 1 %).
+  const int nq = d.nx / V;
+  constexpr int kMaxGrid = 65535;   // y and z blocks of a launch
+  const bool flat = nq % (V == 1 ? 32 : 16) != 0 || d.ny / 8 >= kMaxGrid / 2;
+  cfg.blockDim = V == 4 ? dim3(16, 4) : V == 2 ? dim3(16, 8) : dim3(32, 4);
+  if (flat) {
+    cfg.blockDim = V == 4 ? 64 : 128;
+    cfg.gridDim = dim3((nq * d.ny + cfg.blockDim.x - 1) / cfg.blockDim.x);
+  } else {
+    cfg.gridDim = dim3(nq / cfg.blockDim.x, (d.ny + cfg.blockDim.y - 1) / cfg.blockDim.y);
+  }
+  for (int k0 = 0; k0 < d.nz; k0 += kMaxGrid) {   // one launch, but for grids of more than 65535 levels
+    cfg.gridDim.z = d.nz - k0 < kMaxGrid ? d.nz - k0 : kMaxGrid;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_acoustic_vec<V>, d, ph, c, in, out, dtau, rev, (int)flat, k0);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 cudaError_t launch_acoustic(const Dims& d, const Phys& ph, const Cols& c, AcousticIn in, AcousticOut out, float dtau,
                             cudaStream_t st, int rev, const cudaAccessPolicyWindow* win) {
-  constexpr int VW = ACOUSTIC_VEC;
-#if ACOUSTIC_ZMARCH > 0
-  if (d.nx % VW == 0) {
-    const int nq = d.nx / VW, kc = ACOUSTIC_ZMARCH;
-    dim3 b(16, 16, 1);
-    dim3 g((nq + b.x - 1) / b.x, (d.ny + b.y - 1) / b.y, (d.nz + kc - 1) / kc);
-    k_acoustic_zm<VW><<<g, b, 0, st>>>(d, ph, c, in, out, dtau, kc);
-    return cudaGetLastError();
-  }
-#endif
-  if (d.nx % VW == 0) {
-    const int nq = d.nx / VW;
-    dim3 b(VW == 4 ? 16 : 32, VW == 4 ? 16 : 8, 1);
-    dim3 g((nq + b.x - 1) / b.x, (d.ny + b.y - 1) / b.y, d.nz);
-    if (win) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = g;
-      cfg.blockDim = b;
-      cfg.stream = st;
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeAccessPolicyWindow;
-      at[0].val.accessPolicyWindow = *win;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      return cudaLaunchKernelEx(&cfg, k_acoustic_vec<VW>, d, ph, c, in, out, dtau, rev);
-    }
-    k_acoustic_vec<VW><<<g, b, 0, st>>>(d, ph, c, in, out, dtau, rev);
-    return cudaGetLastError();
-  }
-  dim3 g((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, (d.nz + BZ - 1) / BZ);
-  k_acoustic<<<g, dim3(BX, BY, BZ), 0, st>>>(d, ph, c, in, out, dtau);
-  return cudaGetLastError();
+  if (d.nx % 4 == 0) return launch_vec<4>(d, ph, c, in, out, dtau, st, rev, win);
+  if (d.nx % 2 == 0) return launch_vec<2>(d, ph, c, in, out, dtau, st, rev, win);
+  return launch_vec<1>(d, ph, c, in, out, dtau, st, rev, win);
 }
 
 // Levels per block: enough chunks that the grid fills two blocks per SM.

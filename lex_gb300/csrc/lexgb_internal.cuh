@@ -79,6 +79,12 @@ struct Phys {
   float f_cor;
 };
 
+// Programmatic dependent launch: pdl_wait returns when the previous kernel of the stream has finished
+// and its writes are visible; pdl_trigger lets the next one be scheduled (its blocks start, and wait,
+// as soon as this grid's blocks all run).  Every kernel launched with pdl_attribute waits first.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ int wrap(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
 __device__ __forceinline__ int clampi(int i, int lo, int hi) { return i < lo ? lo : (i > hi ? hi : i); }
 
@@ -256,6 +262,19 @@ __device__ __forceinline__ float buoyancy_at(float T, float q, int k, const Cols
 // ---------------------------------------------------------------------------------------------
 // kernel launchers (stream-ordered; return cudaGetLastError())
 // ---------------------------------------------------------------------------------------------
+inline cudaLaunchAttribute pdl_attribute() {
+  cudaLaunchAttribute a = {};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  return a;
+}
+inline cudaLaunchAttribute window_attribute(const cudaAccessPolicyWindow& w) {
+  cudaLaunchAttribute a = {};
+  a.id = cudaLaunchAttributeAccessPolicyWindow;
+  a.val.accessPolicyWindow = w;
+  return a;
+}
+
 struct State {
   float* T;   // theta - theta_ref
   float* u;
@@ -285,11 +304,11 @@ struct Sgs {
 
 cudaError_t launch_div_trho(const Dims&, const Phys&, const Cols&, State in, float* div, float* trho, cudaStream_t);
 // div_out / trho_out: when given, the divergence div(rho0 u) and theta_rho of `in` are computed here
-// (inside the vertical-march kernel where it runs, else by launch_div_trho first) and `div` is unused
+// and `div` is unused
 cudaError_t launch_adv_scalars(const Dims&, const Phys&, const Cols&, State in, const float* div, const float* T0,
                                const float* q0, Sgs sgs, float dts, SlowOut out, cudaStream_t,
                                float* div_out = nullptr, float* trho_out = nullptr);
-// once per process, before the first launch (opts the momentum kernel into > 48 KB of shared memory)
+// once per process, before the first launch (resident blocks, which the level chunks follow)
 cudaError_t init_weno_attributes();
 // u, v, w together; wmode 0: R_w = adv_w + b8w + sgs_w; 1: adv_w only; 2: b8w only
 cudaError_t launch_adv_momentum(const Dims&, const Phys&, const Cols&, State in, const float* div, Sgs sgs, float* Ru,

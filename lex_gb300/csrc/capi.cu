@@ -385,16 +385,25 @@ extern "C" {
 // fields): a persisting L2 window over them (up to the device's set-aside maximum) keeps them
 // on chip across the 16 or 32 sub-steps, so only the moving state streams through HBM.  The
 // set-aside is a limit of this process's context; failures leave normal caching.
+//
+// Only where the four fields take at most half of the L2: the set-aside is lost to everything else.
+// Measured per big step with and without (us): 192x192x96 (57 MB) 2107 and 2185, 208x208x104 (73 MB)
+// 3062 and 3053, 224x224x112 (90 MB) 4132 and 3584, 240x240x120 (111 MB) 5512 and 4867.
+static bool l2_window_pays(int dev, size_t bytes) {
+  int l2 = 0;
+  return cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) == cudaSuccess && bytes <= (size_t)l2 / 2;
+}
+
 static void setup_l2_window(lexgb_ctx* c) {
+  size_t bytes = 4 * c->fstride * sizeof(float);   // R_u, R_v, R_w, theta_rho
   int dev = 0, max_persist = 0, max_window = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
+  if (cudaGetDevice(&dev) != cudaSuccess || !l2_window_pays(dev, bytes) ||
       cudaDeviceGetAttribute(&max_persist, cudaDevAttrMaxPersistingL2CacheSize, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&max_window, cudaDevAttrMaxAccessPolicyWindowSize, dev) != cudaSuccess ||
       max_persist <= 0 || max_window <= 0) {
     cudaGetLastError();
     return;
   }
-  size_t bytes = 4 * c->fstride * sizeof(float);   // R_u, R_v, R_w, theta_rho
   if (bytes > (size_t)max_window) bytes = (size_t)max_window;
   size_t setaside = bytes < (size_t)max_persist ? bytes : (size_t)max_persist;
   size_t cur = 0;

@@ -282,6 +282,21 @@ int lexgb_cnn_gelu_bwd(long long npts, int c, int cpad, const float *dy, const f
                        void *stream);
 int lexgb_cnn_conv3d_dw(int nx, int ny, int nz, int cin, int cout, int gstride, const void *x, const void *g,
                         float *dw, float *db, void *stream);
+/* One training pass of the network (5 -> 32 -> 32 -> 32 -> 5; npts = nx ny nz points, nx a multiple of
+ * 16) in one call each way.  w: the layers' BF16 weights [27][cout][cin] with (cin, cout) = (16, 32),
+ * (32, 32), (32, 32), (32, 8); b: FP32 biases.
+ * lexgb_cnn_net_forward: x [npts][5] FP32 (NULL: act[0] holds the input already, [npts][16] BF16 with
+ *   zero padding channels) -> out [npts][5] FP32; kept for the backward pass: act[0] [npts][16], act[1..3]
+ *   [npts][32] BF16 (each layer's input) and pre[0..2] [npts][32] FP32 (pre-activations).
+ * lexgb_cnn_net_backward: gout [npts][5] FP32 -> dx [npts][5] FP32 and grads (FP32, overwritten): dw of
+ *   the four layers in w's layout, then db (32, 32, 32, 8).  work: (64 npts + 82944) BF16 of scratch,
+ *   16-byte aligned.  Each layer's input gradient takes GELU' of the layer below and that layer's bias
+ *   sums in the convolution's epilogue. */
+int lexgb_cnn_net_forward(int nx, int ny, int nz, const float *x, const void *const w[4], const float *const b[4],
+                          void *const act[4], float *const pre[3], float *out, void *stream);
+int lexgb_cnn_net_backward(int nx, int ny, int nz, const float *gout, const void *const w[4],
+                           const void *const act[4], const float *const pre[3], void *work, float *grads, float *dx,
+                           void *stream);
 int lexgb_cnn_adam(long long n, float *w, const float *gw, float *m, float *v, void *w_bf16, float lr, float beta1,
                    float beta2, float eps, int step, void *stream);
 

@@ -272,14 +272,14 @@ int run_sgs(lexgb_ctx* c) {
   // programmatic dependent launches only on a created stream (the step graph is captured on the
   // context's own stream); on the legacy or per-thread default stream, plain stream order
   const bool pdl = c->stream != nullptr && c->stream != cudaStreamLegacy && c->stream != cudaStreamPerThread;
-  CK(launch_sgs_pack(d.nx, d.ny, d.nz, c->A.T, c->A.u, c->A.v, c->A.w, c->A.q, (float)c->theta_ref, c->sgs_lo,
-                     c->sgs_rin, c->sgs_x, c->stream));
+  // programmatic dependents: the weights and biases are the context's copies, written only by
+  // lexgb_set_sgs_net, so each layer stages them while the previous kernel finishes
+  CK(launch_sgs_input(d.nx, d.ny, d.nz, c->A.T, c->A.u, c->A.v, c->A.w, c->A.q, (float)c->theta_ref, c->sgs_lo,
+                      c->sgs_rin, c->sgs_x, c->sgs_w[0], c->sgs_b[0], c->sgs_a0, c->stream, pdl));
   const void* in[4] = {c->sgs_x, c->sgs_a0, c->sgs_a1, c->sgs_a0};
   void* out[3] = {c->sgs_a0, c->sgs_a1, c->sgs_a0};
-  for (int l = 0; l < 4; ++l) {
+  for (int l = 1; l < 4; ++l) {
     const bool last = l == 3;
-    // programmatic dependents: the weights and biases are the context's copies, written only by
-    // lexgb_set_sgs_net, so each layer stages them while the previous kernel finishes
     CK(launch_cnn_conv3d(d.nx, d.ny, d.nz, SGS_CIN[l], SGS_COUT[l], in[l], c->sgs_w[l], c->sgs_b[l], nullptr,
                          last ? nullptr : out[l], last ? c->sgs_corr : nullptr, last ? 0 : 1, last ? 5 : SGS_COUT[l],
                          c->stream, pdl));

@@ -23,6 +23,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "lexgb_cnn.cuh"
 
 namespace lexgb {
@@ -44,13 +46,6 @@ __device__ __forceinline__ float gelu_tanh_fast(float x) {
   const float k0 = 0.7978845608028654f;  // sqrt(2/pi)
   return 0.5f * x * (1.f + tanh_fast(k0 * (x + 0.044715f * x * x * x)));
 }
-__device__ __forceinline__ float gelu_tanh_grad(float x) {
-  const float k0 = 0.7978845608028654f;
-  const float u = k0 * (x + 0.044715f * x * x * x);
-  const float t = tanhf(u);
-  return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * k0 * (1.f + 3.f * 0.044715f * x * x);
-}
-
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
@@ -166,14 +161,157 @@ struct ConvSmem {
   static constexpr int A_BYTES = 3 * (CONV_TY + 2) * 18 * CP * 2;
   static constexpr int PS = COUT + 4;                          // partial-sum row stride (floats)
   static constexpr int P_BYTES = CONV_TY * 16 * PS * 4;         // [128 points][PS]
-  static constexpr size_t BYTES = (size_t)W_ELEMS * 2 + (A_BYTES > P_BYTES ? A_BYTES : P_BYTES);
+  // buffers of partial sums: one a plane where two blocks still share an SM, else for planes 0 and 1
+  static constexpr int NB = (size_t)W_ELEMS * 2 + 3 * P_BYTES <= 112 * 1024 ? 3 : 2;
+  static constexpr size_t BYTES = (size_t)W_ELEMS * 2 + (A_BYTES > NB * P_BYTES ? A_BYTES : NB * P_BYTES);
+};
+
+// The weights, [27 COUT][CIN + 8], by the block: 16-byte pieces in the order of both memories, each block
+// from another part of them on, as all blocks read the same ones (a correction at 32^3: 0.9 us)
+template <int CIN, int COUT, int THREADS>
+__device__ __forceinline__ void stage_taps(__nv_bfloat16* ws, const __nv_bfloat16* w) {
+  constexpr int CH = CIN / 8, RT = THREADS / CH, N = 27 * COUT;
+  constexpr int NI = (N + RT - 1) / RT;
+  const int row = (int)(threadIdx.x / CH), c = (int)(threadIdx.x % CH);
+  __nv_bfloat16* const d = ws + row * (CIN + 8) + c * 8;
+  const __nv_bfloat16* const g = w + row * CIN + c * 8;
+  int k = (int)(blockIdx.x % NI);
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    if (row + k * RT < N) cp_async16(d + k * RT * (CIN + 8), g + k * RT * CIN, true);
+    if (++k == NI) k = 0;
+  }
+}
+
+// One input plane of a tile with its halo, [CONV_TY + 2][18][CIN + 8], zero outside the grid, by the
+// CONV_RP warps that read it: thread t of 32 CONV_RP, 16-byte pieces in the order of both memories
+template <int CIN>
+__device__ __forceinline__ void stage_plane(__nv_bfloat16* ap, const __nv_bfloat16* x, int nx, int ny, int nz, int x0,
+                                            int y0, int zz, unsigned t) {
+  constexpr int CH = CIN / 8, RT = 32 * CONV_RP / CH, N = (CONV_TY + 2) * 18;
+  const bool inz = zz >= 0 && zz < nz;
+  const int c = (int)(t % CH);
+  int q = (int)(t / CH), hy = q / 18, hx = q - 18 * hy;
+  const __nv_bfloat16* const xp = x + (((long long)(inz ? zz : 0) * ny + y0 - 1) * nx + x0 - 1) * CIN + c * 8;
+  __nv_bfloat16* const d = ap + q * (CIN + 8) + c * 8;
+#pragma unroll
+  for (int i = 0; i < (N + RT - 1) / RT; ++i) {
+    if ((i + 1) * RT <= N || q + i * RT < N) {
+      const bool in = inz && (unsigned)(x0 + hx - 1) < (unsigned)nx && (unsigned)(y0 + hy - 1) < (unsigned)ny;
+      cp_async16(d + i * RT * (CIN + 8), in ? xp + (hy * nx + hx) * CIN : x, in);
+    }
+    hx += RT % 18;
+    hy += RT / 18;
+    if (hx >= 18) hx -= 18, ++hy;
+  }
+}
+
+// (a + *b) + *c
+__device__ __forceinline__ float4 sum3(float4 a, const float* b, const float* c) {
+  const float4 u = *reinterpret_cast<const float4*>(b), v = *reinterpret_cast<const float4*>(c);
+  return make_float4((a.x + u.x) + v.x, (a.y + u.y) + v.y, (a.z + u.z) + v.z, (a.w + u.w) + v.w);
+}
+
+// The epilogue of a tile of 16 x CONV_TY points over a whole block: four channels of a point at a time
+// (a thread's channels are the same in every pass).
+template <int COUT, int THREADS, int LV = 1>
+struct ConvEpi {
+  static constexpr int CPP = COUT / 4, PTS = LV * CONV_TY * 16, IT = (PTS * CPP + THREADS - 1) / THREADS;
+  int co;
+  float4 b4, db;   // the thread's biases, its sums for ConvEpilogue::db
+  bool vec;        // 16-byte aligned outputs
+  __device__ __forceinline__ explicit ConvEpi(const ConvEpilogue& o) : co((int)(4 * (threadIdx.x % CPP))) {
+    b4 = o.bias ? make_float4(o.bias[co], o.bias[co + 1], o.bias[co + 2], o.bias[co + 3])
+                : make_float4(0.f, 0.f, 0.f, 0.f);
+    db = make_float4(0.f, 0.f, 0.f, 0.f);
+    vec = (((uintptr_t)o.pre | (uintptr_t)o.yf | (uintptr_t)o.gpre | (uintptr_t)o.ybf) & 15) == 0;
+  }
+  __device__ __forceinline__ void st4(float* d, float4 v) const {
+    if (vec) {
+      *reinterpret_cast<float4*>(d) = v;
+    } else {
+      d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+    }
+  }
+  __device__ __forceinline__ float4 ld4(const float* d) const {
+    return vec ? __ldg(reinterpret_cast<const float4*>(d)) : make_float4(d[0], d[1], d[2], d[3]);
+  }
+  // sum(pt, channel): the convolution's four sums at point pt of the tile's LV levels
+  template <class F>
+  __device__ __forceinline__ void tile(const ConvEpilogue& o, int nx, int ny, int nz, int x0, int y0, int z, const F& sum) {
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      const unsigned pt = threadIdx.x / CPP + i * (THREADS / CPP);
+      const int y = y0 + (int)(pt / 16 % CONV_TY), zl = z + (LV > 1 ? (int)(pt / (16 * CONV_TY)) : 0);
+      if (pt >= PTS || y >= ny || zl >= nz) continue;
+      // two levels: a grid of at most two tiles an SM
+      const std::conditional_t<(LV > 1), int, long long> row = (std::conditional_t<(LV > 1), int, long long>)zl * ny + y;
+      const long long p = row * nx + x0 + (int)(pt % 16);
+      float4 gp = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (o.gpre) gp = ld4(o.gpre + p * COUT + co);
+      float4 a = sum(pt, co);
+      a = make_float4(a.x + b4.x, a.y + b4.y, a.z + b4.z, a.w + b4.w);
+      if (o.pre) st4(o.pre + p * COUT + co, a);
+      if (o.gelu) a = make_float4(gelu_tanh_fast(a.x), gelu_tanh_fast(a.y), gelu_tanh_fast(a.z), gelu_tanh_fast(a.w));
+      if (o.gpre)
+        a = make_float4(a.x * gelu_tanh_grad(gp.x), a.y * gelu_tanh_grad(gp.y), a.z * gelu_tanh_grad(gp.z),
+                        a.w * gelu_tanh_grad(gp.w));
+      if (co + 3 >= o.creal) {
+        if (co >= o.creal) a.x = 0.f;
+        if (co + 1 >= o.creal) a.y = 0.f;
+        if (co + 2 >= o.creal) a.z = 0.f;
+        a.w = 0.f;
+      }
+      if (o.ybf) {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
+        __nv_bfloat16* const d = reinterpret_cast<__nv_bfloat16*>(o.ybf) + p * COUT + co;
+        if (vec) {
+          uint2 qq;
+          qq.x = *reinterpret_cast<const uint32_t*>(&lo);
+          qq.y = *reinterpret_cast<const uint32_t*>(&hi);
+          *reinterpret_cast<uint2*>(d) = qq;
+        } else {
+          reinterpret_cast<__nv_bfloat162*>(d)[0] = lo;
+          reinterpret_cast<__nv_bfloat162*>(d)[1] = hi;
+        }
+        const float2 l = __bfloat1622float2(lo), h = __bfloat1622float2(hi);
+        db = make_float4(db.x + l.x, db.y + l.y, db.z + h.x, db.w + h.y);
+      }
+      if (o.yf && !o.compact) {
+        st4(o.yf + p * COUT + co, a);
+      } else if (o.yf) {
+        float* const d = o.yf + p * o.creal + co;
+        if (co < o.creal) d[0] = a.x;
+        if (co + 1 < o.creal) d[1] = a.y;
+        if (co + 2 < o.creal) d[2] = a.z;
+        if (co + 3 < o.creal) d[3] = a.w;
+      }
+    }
+  }
+  // the block's sums: lanes with the same channels, then one addition a warp and channel
+  __device__ __forceinline__ void finish(const ConvEpilogue& o) {
+    if (!o.db) return;
+#pragma unroll
+    for (int m = CPP; m < 32; m *= 2) {
+      db.x += __shfl_xor_sync(0xffffffffu, db.x, m);
+      db.y += __shfl_xor_sync(0xffffffffu, db.y, m);
+      db.z += __shfl_xor_sync(0xffffffffu, db.z, m);
+      db.w += __shfl_xor_sync(0xffffffffu, db.w, m);
+    }
+    const int lane = threadIdx.x & 31;
+    if (lane < CPP) {
+      atomicAdd(o.db + 4 * lane, db.x);
+      atomicAdd(o.db + 4 * lane + 1, db.y);
+      atomicAdd(o.db + 4 * lane + 2, db.z);
+      atomicAdd(o.db + 4 * lane + 3, db.w);
+    }
+  }
 };
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(ConvSmem<CIN, COUT>::THREADS)
     k_conv3d_smem(int nx, int ny, int nz, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                  const float* __restrict__ bias, float* __restrict__ pre, __nv_bfloat16* __restrict__ ybf,
-                  float* __restrict__ yf, int gelu, int creal, int early_weights) {
+                  const ConvEpilogue o, int early_weights) {
   using L = ConvSmem<CIN, COUT>;
   constexpr int CP = L::CP, NT = L::NT, KC = CIN / 16, CH = CIN / 8;  // CH: 16-byte chunks a row
   extern __shared__ __align__(16) __nv_bfloat16 conv_smem[];
@@ -187,10 +325,7 @@ __global__ void __launch_bounds__(ConvSmem<CIN, COUT>::THREADS)
   // read only after pdl_wait
   pdl_launch_dependents();
   if (!early_weights) pdl_wait();
-  for (int e = tid; e < 27 * COUT * CH; e += L::THREADS) {
-    const int row = e / CH, c = e % CH;
-    cp_async16(Ws + row * CP + c * 8, w + (long long)row * CIN + c * 8, true);
-  }
+  stage_taps<CIN, COUT, L::THREADS>(Ws, w);
   if (early_weights) pdl_wait();
   const int tiles_x = nx / 16, tiles_y = (ny + CONV_TY - 1) / CONV_TY;
   const long long ntiles = (long long)tiles_x * tiles_y * nz;
@@ -199,18 +334,13 @@ __global__ void __launch_bounds__(ConvSmem<CIN, COUT>::THREADS)
   const int a_row = ((lane >> 3) & 1) * 8 + (lane & 7), a_k = (lane >> 4) * 8;
   // B (x4, two n8 tiles): matrix m -> tile m >> 1, k half m & 1; (x2) matrix m -> k half m
   const int b_row = (lane >> 4) * 8 + (lane & 7), b_k = ((lane >> 3) & 1) * 8;
+  ConvEpi<COUT, L::THREADS> ep(o);
   for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int tx = (int)(tile % tiles_x), ty = (int)((tile / tiles_x) % tiles_y);
     const int z = (int)(tile / ((long long)tiles_x * tiles_y));
     const int x0 = tx * 16, y0 = ty * CONV_TY;
     __syncthreads();  // the previous tile's reads of As / Ps are done
-    for (int e = tid; e < 3 * (CONV_TY + 2) * 18 * CH; e += L::THREADS) {
-      const int c = e % CH, q = e / CH;
-      const int hx = q % 18, hy = (q / 18) % (CONV_TY + 2), hz = q / (18 * (CONV_TY + 2));
-      const int xx = x0 + hx - 1, yy = y0 + hy - 1, zz = z + hz - 1;
-      const bool in = xx >= 0 && xx < nx && yy >= 0 && yy < ny && zz >= 0 && zz < nz;
-      cp_async16(As + q * CP + c * 8, in ? x + (((long long)zz * ny + yy) * nx + xx) * CIN + c * 8 : x, in);
-    }
+    stage_plane<CIN>(As + dz * (CONV_TY + 2) * 18 * CP, x, nx, ny, nz, x0, y0, z + dz - 1, rp * 32 + lane);
     cp_async_wait_all();
     __syncthreads();
     const int ya = y0 + rp, yb = ya + CONV_RP;  // the warp's two rows
@@ -260,47 +390,243 @@ __global__ void __launch_bounds__(ConvSmem<CIN, COUT>::THREADS)
       }
     }
     __syncthreads();  // every warp is done with As: it becomes the partial sums [point][channel]
-    // planes added in order: plane 0 writes (zeros where it does not exist), 1 and 2 add
-    constexpr int PS = L::PS;
-#pragma unroll 1
-    for (int d = 0; d < 3; ++d) {
-      if (dz == d && (d == 0 || (plane && ya < ny))) {
+    // the planes' sums meet as (plane 0 + plane 1) + plane 2 (zeros where a plane does not exist):
+    // in the epilogue, or with two buffers plane 2's warps add theirs to the other two
+    constexpr int PS = L::PS, PB = CONV_TY * 16 * PS;
+    auto each = [&](const auto& f) {
 #pragma unroll
-        for (int m = 0; m < CONV_MR; ++m)
+      for (int m = 0; m < CONV_MR; ++m)
 #pragma unroll
-          for (int n = 0; n < NT; ++n)
+        for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              float2* pp = reinterpret_cast<float2*>(Ps + ((rp + m * CONV_RP) * 16 + g + 8 * h) * PS + n * 8 + 2 * t);
-              float2 v = make_float2(acc[m][n][2 * h], acc[m][n][2 * h + 1]);
-              if (d > 0) {
-                const float2 o = *pp;
-                v = make_float2(o.x + v.x, o.y + v.y);
-              }
-              *pp = v;
-            }
-      }
+          for (int h = 0; h < 2; ++h)
+            f(reinterpret_cast<float2*>(Ps + ((rp + m * CONV_RP) * 16 + g + 8 * h) * PS + n * 8 + 2 * t),
+              make_float2(acc[m][n][2 * h], acc[m][n][2 * h + 1]));
+    };
+    if (dz < L::NB) each([&](float2* d, float2 v) { d[dz * (PB / 2)] = v; });
+    __syncthreads();
+    if (L::NB == 2) {
+      if (dz == 2)
+        each([&](float2* d, float2 v) {
+          const float2 a = d[0], b = d[PB / 2];
+          d[0] = make_float2((a.x + b.x) + v.x, (a.y + b.y) + v.y);
+        });
       __syncthreads();
     }
-    // epilogue over the whole block: channel pairs of the tile's 128 points
-    for (int e = tid; e < CONV_TY * 16 * (COUT / 2); e += L::THREADS) {
-      const int pt = e / (COUT / 2), co = (e % (COUT / 2)) * 2;
-      const int y = y0 + pt / 16;
-      if (y >= ny) continue;
-      const long long p = ((long long)z * ny + y) * nx + x0 + (pt % 16);
-      const float2 sum = *reinterpret_cast<const float2*>(Ps + pt * PS + co);
-      float v0 = sum.x + (bias ? bias[co] : 0.f), v1 = sum.y + (bias ? bias[co + 1] : 0.f);
-      if (pre) *reinterpret_cast<float2*>(pre + p * COUT + co) = make_float2(v0, v1);
-      if (gelu) {
-        v0 = gelu_tanh_fast(v0);
-        v1 = gelu_tanh_fast(v1);
-      }
-      if (co >= creal) v0 = 0.f;
-      if (co + 1 >= creal) v1 = 0.f;
-      if (ybf) *reinterpret_cast<__nv_bfloat162*>(ybf + p * COUT + co) = __floats2bfloat162_rn(v0, v1);
-      if (yf) *reinterpret_cast<float2*>(yf + p * COUT + co) = make_float2(v0, v1);
-    }
+    ep.tile(o, nx, ny, nz, x0, y0, z, [&](int pt, int c) {
+      const float* const r = Ps + pt * PS + c;
+      const float4 a = *reinterpret_cast<const float4*>(r);
+      return L::NB == 3 ? sum3(a, r + PB, r + 2 * PB) : a;
+    });
   }
+  ep.finish(o);
+}
+
+// The same convolution, two levels a block, once over the grid: where that gives each SM one block, the
+// weights cross once a block instead of once a level, the levels share two of their four input planes,
+// and a warp's A fragments feed both levels: 32^3, 9.1 -> 7.7 us a layer 16 -> 32, 11.5 -> 9.7 (32 -> 32),
+// 6.8 -> 5.5 (32 -> 8).  Of the 9.7 us the products take 4.1 (one mma.sync in 8 cycles a scheduler is the
+// tensor pipe's rate, 3.6 us here), staging 2.2, the sums and the epilogue 2.3, one after another with one
+// block an SM.  Warp (p, r) takes input plane z0 + p - 1 for the levels it feeds; the sums are those of
+// k_conv3d_smem, bit for bit.  PACK (16 -> 32): the input made from the state where it is staged, for the
+// halo too, in place of a kernel that writes it: 2.0 us of a correction.
+template <int CIN, int COUT>
+struct ConvSmem2 {
+  using S = ConvSmem<CIN, COUT>;
+  static constexpr int PS = COUT == 8 ? 12 : COUT + 8;   // floats a point of partial sums: stores of 8 bytes in distinct banks
+  static constexpr int WARPS = 4 * CONV_RP, THREADS = 32 * WARPS;
+  static constexpr size_t A_BYTES = (size_t)4 * (CONV_TY + 2) * 18 * S::CP * 2;
+  static constexpr size_t IN = (size_t)S::W_ELEMS * 2 + A_BYTES, OUT = (size_t)6 * CONV_TY * 16 * PS * 4;   // OUT over IN
+  static constexpr size_t BYTES = IN > OUT ? IN : OUT;
+};
+
+template <int CIN, int COUT, bool PACK>
+__global__ void __launch_bounds__(ConvSmem2<CIN, COUT>::THREADS)
+    k_conv3d_smem2(int nx, int ny, int nz, const __nv_bfloat16* __restrict__ x, const PackIn in,
+                   const __nv_bfloat16* __restrict__ w, const ConvEpilogue o, int early_weights) {
+  using L = ConvSmem2<CIN, COUT>;
+  using S1 = ConvSmem<CIN, COUT>;
+  constexpr int CP = S1::CP, NT = S1::NT, KC = CIN / 16, CH = CIN / 8, PS = L::PS, PB = CONV_TY * 16 * PS;
+  extern __shared__ __align__(16) __nv_bfloat16 conv_smem[];
+  __nv_bfloat16* Ws = conv_smem;
+  __nv_bfloat16* As = conv_smem + S1::W_ELEMS;
+  float* Ps = reinterpret_cast<float*>(conv_smem);   // partial sums [level][tap plane], over everything
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int pl = wid / CONV_RP, rp = wid % CONV_RP;
+  pdl_launch_dependents();
+  if (!early_weights) pdl_wait();
+  stage_taps<CIN, COUT, L::THREADS>(Ws, w);
+  ConvEpi<COUT, L::THREADS, 2> ep(o);
+  const int tiles_x = nx / 16, tiles_y = (ny + CONV_TY - 1) / CONV_TY;
+  const int tx = blockIdx.x % tiles_x, ty = (blockIdx.x / tiles_x) % tiles_y;
+  const int x0 = tx * 16, y0 = ty * CONV_TY, z0 = 2 * (blockIdx.x / (tiles_x * tiles_y));
+  std::conditional_t<PACK, PackNorm, int> nrm{};
+  if constexpr (PACK) nrm = PackNorm(in, min(max(z0 + pl - 1, 0), nz - 1), nz);   // constant, like the weights
+  if (early_weights) pdl_wait();
+  __nv_bfloat16* const ap = As + pl * (CONV_TY + 2) * 18 * CP;
+  if constexpr (PACK) {
+    const int zz = z0 + pl - 1;
+    constexpr int PTS = (CONV_TY + 2) * 18, T = 32 * CONV_RP, IT = (PTS + T - 1) / T;
+    const bool inz = zz >= 0 && zz < nz;
+    PackPoint f[IT];
+    bool ok[IT];
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      const int e = rp * 32 + lane + i * T, xx = x0 + e % 18 - 1, yy = y0 + e / 18 - 1;
+      ok[i] = inz && e < PTS && xx >= 0 && xx < nx && yy >= 0 && yy < ny;
+      if (ok[i]) f[i].load(in, xx, yy, zz, nx, ny);
+    }
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      const int e = rp * 32 + lane + i * T;
+      if (e >= PTS) continue;
+      uint4* const d = reinterpret_cast<uint4*>(ap + e * CP);
+      d[0] = ok[i] ? f[i].channels(in, nrm) : make_uint4(0u, 0u, 0u, 0u);
+      d[1] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  } else {
+    stage_plane<CIN>(ap, x, nx, ny, nz, x0, y0, z0 + pl - 1, rp * 32 + lane);
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  const int g = lane >> 2, t = lane & 3;
+  const int a_row = ((lane >> 3) & 1) * 8 + (lane & 7), a_k = (lane >> 4) * 8;
+  const int b_row = (lane >> 4) * 8 + (lane & 7), b_k = ((lane >> 3) & 1) * 8;
+  const int ya = y0 + rp, yb = ya + CONV_RP;
+  float acc[2][CONV_MR][NT][4];
+#pragma unroll
+  for (int l = 0; l < 2; ++l)
+#pragma unroll
+    for (int m = 0; m < CONV_MR; ++m)
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[l][m][n][q] = 0.f;
+  // the products of a plane that feeds levels LA..LB
+  auto products = [&](auto la, auto lb) {
+    constexpr int LA = decltype(la)::value, LB = decltype(lb)::value;
+#pragma unroll 1
+    for (int dy = 0; dy < 3; ++dy) {
+      const bool ina = ya + dy - 1 >= 0 && ya + dy - 1 < ny, inb = yb + dy - 1 >= 0 && yb + dy - 1 < ny;
+      if (!ina && !inb) continue;
+      const __nv_bfloat16* arow = As + ((pl * (CONV_TY + 2) + rp + dy) * 18 + a_row) * CP + a_k;
+      const __nv_bfloat16* wrow = Ws + ((pl * 9 + dy * 3) * COUT + (NT == 1 ? lane & 7 : b_row)) * CP + b_k;
+      if constexpr (NT == 1) {   // few products: every load first
+        uint32_t a[3 * KC][CONV_MR][4], b[3 * KC][2][2];
+#pragma unroll
+        for (int i = 0; i < 3 * KC; ++i) {
+#pragma unroll
+          for (int m = 0; m < CONV_MR; ++m)
+            ldsm_x4(a[i][m], arow + (m * CONV_RP * 18 + i / KC) * CP + i % KC * 16);
+#pragma unroll
+          for (int l = LA; l <= LB; ++l) ldsm_x2(b[i][l], wrow + (i / KC - 9 * l) * COUT * CP + i % KC * 16);
+        }
+#pragma unroll
+        for (int i = 0; i < 3 * KC; ++i)
+#pragma unroll
+          for (int l = LA; l <= LB; ++l)
+#pragma unroll
+            for (int m = 0; m < CONV_MR; ++m) mma_bf16(acc[l][m][0], a[i][m], b[i][l]);
+        continue;
+      }
+#pragma unroll
+      for (int dx = 0; dx < 3; ++dx) {
+#pragma unroll
+        for (int kc = 0; kc < KC; ++kc) {
+          uint32_t a[CONV_MR][4];
+#pragma unroll
+          for (int m = 0; m < CONV_MR; ++m) ldsm_x4(a[m], arow + (m * CONV_RP * 18 + dx) * CP + kc * 16);
+#pragma unroll
+          for (int l = LA; l <= LB; ++l) {   // the plane is tap dz = pl - l of level z0 + l
+            const __nv_bfloat16* wo = wrow + (dx - 9 * l) * COUT * CP + kc * 16;
+#pragma unroll
+            for (int n2 = 0; n2 < NT / 2; ++n2) {
+              uint32_t b4[4];
+              ldsm_x4(b4, wo + n2 * 16 * CP);
+              const uint32_t b0[2] = {b4[0], b4[1]}, b1[2] = {b4[2], b4[3]};
+#pragma unroll
+              for (int m = 0; m < CONV_MR; ++m) {
+                mma_bf16(acc[l][m][2 * n2], a[m], b0);
+                mma_bf16(acc[l][m][2 * n2 + 1], a[m], b1);
+              }
+            }
+          }
+        }
+      }
+    }
+  };
+  if (z0 + pl - 1 >= 0 && z0 + pl - 1 < nz && ya < ny) {
+    constexpr std::integral_constant<int, 0> lo{};
+    constexpr std::integral_constant<int, 1> hi{};
+    if (pl == 0)
+      products(lo, lo);
+    else if (pl == 3)
+      products(hi, hi);
+    else
+      products(lo, hi);
+  }
+  __syncthreads();   // every warp is done with the weights and planes: the partial sums replace them
+#pragma unroll
+  for (int l = 0; l < 2; ++l) {
+    const int dz = pl - l;
+    if (dz < 0 || dz > 2) continue;
+    float* const d = Ps + (l * 3 + dz) * PB;
+#pragma unroll
+    for (int m = 0; m < CONV_MR; ++m)
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          *reinterpret_cast<float2*>(d + ((rp + m * CONV_RP) * 16 + g + 8 * h) * PS + n * 8 + 2 * t) =
+              make_float2(acc[l][m][n][2 * h], acc[l][m][n][2 * h + 1]);
+  }
+  __syncthreads();
+  ep.tile(o, nx, ny, nz, x0, y0, z0, [&](int pt, int c) {
+    const float* const r = Ps + (pt / (16 * CONV_TY)) * 2 * PB + pt * PS + c;
+    return sum3(*reinterpret_cast<const float4*>(r), r + PB, r + 2 * PB);
+  });
+  ep.finish(o);
+}
+
+// [npts][5] FP32 -> [npts][16] BF16, the padding zero: the network's input, and the gradient at its
+// output; db (8 channels) += the sums of the rounded values.
+__global__ void __launch_bounds__(256) k_pad5(long long npts, const float* __restrict__ in, uint4* __restrict__ out,
+                                              float* __restrict__ db) {
+  float s[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < npts; p += (long long)gridDim.x * blockDim.x) {
+    unsigned short h[6];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      const __nv_bfloat16 b = __float2bfloat16_rn(__ldg(in + p * 5 + c));
+      h[c] = __bfloat16_as_ushort(b);
+      s[c] += __bfloat162float(b);
+    }
+    out[2 * p] = make_uint4(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16, h[4], 0u);
+    out[2 * p + 1] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (!db) return;
+#pragma unroll
+  for (int c = 0; c < 5; ++c) {
+#pragma unroll
+    for (int m = 16; m > 0; m /= 2) s[c] += __shfl_xor_sync(0xffffffffu, s[c], m);
+    if ((threadIdx.x & 31) == 0) atomicAdd(db + c, s[c]);
+  }
+}
+
+// The input-gradient weights of the four layers: [27][cout][cin] -> [27][cin][g], offsets reversed,
+// the g gradient channels cout padded with zeros (16 for the last layer's 8).
+struct MirrorArgs {
+  const __nv_bfloat16* w[4];
+  __nv_bfloat16* out[4];
+  int cin[4], cout[4], g[4], end[4];   // end: running total of the outputs
+};
+__global__ void k_mirror(MirrorArgs a) {
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= a.end[3]) return;
+  const int l = t < a.end[0] ? 0 : t < a.end[1] ? 1 : t < a.end[2] ? 2 : 3;
+  if (l) t -= a.end[l - 1];
+  const int co = t % a.g[l], ci = t / a.g[l] % a.cin[l], tap = t / (a.g[l] * a.cin[l]);
+  a.out[l][t] = co < a.cout[l] ? a.w[l][((26 - tap) * a.cout[l] + co) * a.cin[l] + ci] : __float2bfloat16_rn(0.f);
 }
 
 // g[p][c] = dy[p][c] * GELU'(pre[p][c]) for c < C (pre and dy have C channels, FP32), written
@@ -379,45 +705,18 @@ __global__ void k_adam(long long n, float* __restrict__ w, const float* __restri
   if (wbf) wbf[t] = __float2bfloat16(ww);
 }
 
-// Input of the network, one thread per cell, 16 BF16 channels (32 bytes):
-//   (theta, ui, vi, wi, qv, 0 x 11), each (value - lo[f][k]) / rin[f][k]
-// with theta = T + theta_ref and the winds averaged to the cell centre (u, v periodic).  The
-// arithmetic is the element-wise sequence of the PyTorch packing of the same state, rounded
-// the same way (no contractions), so both give the same BF16 inputs.
-// Network input of one cell, as dl_models.phys_state_tuple2array makes it (dl_models.py:125-155):
-// every field is min-max normalised on its own grid points with per-level constants lo[f][l] and
-// rin[f][l] (stride nz+1: w's constants are per face level 0..nz), then the normalised winds are
-// averaged to the cell centre (unstagger_uvw).  16 BF16 channels, 5 used.
-__global__ void k_sgs_pack(int nx, int ny, int nz, const float* __restrict__ T, const float* __restrict__ u,
-                           const float* __restrict__ v, const float* __restrict__ w, const float* __restrict__ q,
-                           float theta_ref, const float* __restrict__ lo, const float* __restrict__ rin,
-                           uint4* __restrict__ x16) {
+// Input of the network (PackPoint), one thread per cell, 16 BF16 channels (32 bytes)
+__global__ void k_sgs_pack(int nx, int ny, int nz, const PackIn in, uint4* __restrict__ x16) {
   pdl_launch_dependents();
+  pdl_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long plane = (long long)nx * ny;
   if (t >= plane * nz) return;
-  const int i = (int)(t % nx), j = (int)((t / nx) % ny), k = (int)(t / plane);
-  const long long tu = t - i + (i + 1 == nx ? 0 : i + 1);
-  const long long tv = t + (long long)((j + 1 == ny ? 0 : j + 1) - j) * nx;
-  const int L = nz + 1;
-  auto nrm = [&](float x, int f, int l) { return __fdiv_rn(__fsub_rn(x, lo[f * L + l]), rin[f * L + l]); };
-  float f[5];
-  f[0] = nrm(__fadd_rn(T[t], theta_ref), 0, k);
-  f[1] = __fmul_rn(0.5f, __fadd_rn(nrm(u[t], 1, k), nrm(u[tu], 1, k)));
-  f[2] = __fmul_rn(0.5f, __fadd_rn(nrm(v[t], 2, k), nrm(v[tv], 2, k)));
-  f[3] = __fmul_rn(0.5f, __fadd_rn(nrm(w[t], 3, k), nrm(w[t + plane], 3, k + 1)));
-  f[4] = nrm(q[t], 4, k);
-  __nv_bfloat16 h[6];
-#pragma unroll
-  for (int c = 0; c < 5; ++c) h[c] = __float2bfloat16_rn(f[c]);
-  h[5] = __float2bfloat16_rn(0.f);
-  uint4 a, b = make_uint4(0u, 0u, 0u, 0u);
-  a.x = (uint32_t)__bfloat16_as_ushort(h[0]) | ((uint32_t)__bfloat16_as_ushort(h[1]) << 16);
-  a.y = (uint32_t)__bfloat16_as_ushort(h[2]) | ((uint32_t)__bfloat16_as_ushort(h[3]) << 16);
-  a.z = (uint32_t)__bfloat16_as_ushort(h[4]) | ((uint32_t)__bfloat16_as_ushort(h[5]) << 16);
-  a.w = 0u;
-  x16[2 * t] = a;
-  x16[2 * t + 1] = b;
+  const int k = (int)(t / plane);
+  PackPoint f;
+  f.load(in, (int)(t % nx), (int)((t / nx) % ny), k, nx, ny);
+  x16[2 * t] = f.channels(in, PackNorm(in, k, nz));
+  x16[2 * t + 1] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 // The correction corr[p][0..4] (FP32, 8 channels a point) back on the grid as
@@ -431,21 +730,23 @@ __global__ void k_sgs_pack(int nx, int ny, int nz, const float* __restrict__ T, 
 __global__ void k_sgs_unpack(int nx, int ny, int nz, const float* __restrict__ corr, const float* __restrict__ rout,
                              float* __restrict__ T, float* __restrict__ u, float* __restrict__ v, float* __restrict__ w,
                              float* __restrict__ q) {
-  pdl_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long plane = (long long)nx * ny, cells = plane * nz, rstride = plane * (nz + 1);
   if (t >= cells) return;
   const int i = (int)(t % nx), j = (int)((t / nx) % ny), k = (int)(t / plane);
-  auto c = [&](long long p, int f) { return corr[p * 8 + f]; };
-  auto r = [&](long long p, int f) { return rout[f * rstride + p]; };
+  float r[5];   // the ranges are the context's copies, like the weights: read while the network finishes
+#pragma unroll
+  for (int f = 0; f < 5; ++f) r[f] = __ldg(rout + f * rstride + t);
   // the two cells beside the west (south) face; face 0 takes cells nx-2, nx-1 (ny-2, ny-1)
   const long long ua = i > 0 ? t - 1 : t + (nx - 2), ub = i > 0 ? t : t + (nx - 1);
   const long long va = j > 0 ? t - nx : t + (long long)(ny - 2) * nx, vb = j > 0 ? t : t + (long long)(ny - 1) * nx;
-  T[t] = __fadd_rn(T[t], __fmul_rn(c(t, 0), r(t, 0)));
-  u[t] = __fadd_rn(u[t], __fmul_rn(__fmul_rn(0.5f, __fadd_rn(c(ua, 1), c(ub, 1))), r(t, 1)));
-  v[t] = __fadd_rn(v[t], __fmul_rn(__fmul_rn(0.5f, __fadd_rn(c(va, 2), c(vb, 2))), r(t, 2)));
-  if (k > 0) w[t] = __fadd_rn(w[t], __fmul_rn(__fmul_rn(0.5f, __fadd_rn(c(t - plane, 3), c(t, 3))), r(t, 3)));
-  q[t] = __fadd_rn(q[t], __fmul_rn(c(t, 4), r(t, 4)));
+  pdl_wait();
+  auto c = [&](long long p, int f) { return corr[p * 8 + f]; };
+  T[t] = __fadd_rn(T[t], __fmul_rn(c(t, 0), r[0]));
+  u[t] = __fadd_rn(u[t], __fmul_rn(__fmul_rn(0.5f, __fadd_rn(c(ua, 1), c(ub, 1))), r[1]));
+  v[t] = __fadd_rn(v[t], __fmul_rn(__fmul_rn(0.5f, __fadd_rn(c(va, 2), c(vb, 2))), r[2]));
+  if (k > 0) w[t] = __fadd_rn(w[t], __fmul_rn(__fmul_rn(0.5f, __fadd_rn(c(t - plane, 3), c(t, 3))), r[3]));
+  q[t] = __fadd_rn(q[t], __fmul_rn(c(t, 4), r[4]));
 }
 }  // namespace
 
@@ -455,37 +756,51 @@ __global__ void k_sgs_unpack(int nx, int ny, int nz, const float* __restrict__ c
 constexpr int CONV_MAX_DEVICES = 64;
 
 template <int CIN, int COUT>
-cudaError_t conv_grid(int* cap) {
-  static int grid_cap[CONV_MAX_DEVICES] = {};
+cudaError_t conv_grid(int* cap, int* nsm) {
+  static int grid_cap[CONV_MAX_DEVICES] = {}, sm_count[CONV_MAX_DEVICES] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= CONV_MAX_DEVICES) return cudaErrorInvalidDevice;
   if (!grid_cap[dev]) {
     using L = ConvSmem<CIN, COUT>;
-    e = cudaFuncSetAttribute(k_conv3d_smem<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES);
-    if (e != cudaSuccess) return e;
+    constexpr cudaFuncAttribute dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    const int two = (int)ConvSmem2<CIN, COUT>::BYTES;
+    if ((e = cudaFuncSetAttribute(k_conv3d_smem<CIN, COUT>, dyn, (int)L::BYTES)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_conv3d_smem2<CIN, COUT, false>, dyn, two)) != cudaSuccess) return e;
+    if constexpr (CIN == 16 && COUT == 32)
+      if ((e = cudaFuncSetAttribute(k_conv3d_smem2<CIN, COUT, true>, dyn, two)) != cudaSuccess) return e;
     int sms = 0, per = 0;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_conv3d_smem<CIN, COUT>, L::THREADS, L::BYTES)) !=
         cudaSuccess)
       return e;
+    sm_count[dev] = sms;
     grid_cap[dev] = sms * (per > 0 ? per : 1);
   }
   *cap = grid_cap[dev];
+  *nsm = sm_count[dev];
   return cudaSuccess;
 }
 
+// One level a block where every block has an SM of its own, two where that still gives each SM one block,
+// else tiles in turn on the resident blocks (a correction at 32^3: 40.0 us in turn, 34.5 in pairs)
+static long long conv_tiles(int nx, int ny, int nz) { return (long long)(nx / 16) * ((ny + CONV_TY - 1) / CONV_TY) * nz; }
+static bool conv_pairs(int nx, int ny, int nz, int sms) {
+  const long long t = conv_tiles(nx, ny, nz);
+  return t > sms && t / nz * ((nz + 1) / 2) <= sms;
+}
+
 // pdl: launch as a programmatic dependent of the previous kernel of the stream, staging the
-// weights before waiting for it (the caller guarantees that kernel does not write them)
+// weights before waiting for it (the caller guarantees that kernel does not write them).  pack: the
+// state the input is made of in place (16 -> 32 channels where conv_pairs).
 template <int CIN, int COUT>
 cudaError_t launch_conv_smem(int nx, int ny, int nz, const __nv_bfloat16* x, const __nv_bfloat16* w,
-                             const float* bias, float* pre, __nv_bfloat16* ybf, float* yf, int gelu, int creal,
-                             cudaStream_t st, bool pdl) {
-  int cap = 0;
-  cudaError_t e = conv_grid<CIN, COUT>(&cap);
+                             const ConvEpilogue& o, cudaStream_t st, bool pdl, const PackIn* pack = nullptr) {
+  int cap = 0, sms = 0;
+  cudaError_t e = conv_grid<CIN, COUT>(&cap, &sms);
   if (e != cudaSuccess) return e;
-  const long long ntiles = (long long)(nx / 16) * ((ny + CONV_TY - 1) / CONV_TY) * nz;
+  const long long ntiles = conv_tiles(nx, ny, nz);
   using L = ConvSmem<CIN, COUT>;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(ntiles < cap ? ntiles : cap));
@@ -497,53 +812,114 @@ cudaError_t launch_conv_smem(int nx, int ny, int nz, const __nv_bfloat16* x, con
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, k_conv3d_smem<CIN, COUT>, nx, ny, nz, x, w, bias, pre, ybf, yf, gelu, creal,
-                            pdl ? 1 : 0);
+  if (!conv_pairs(nx, ny, nz, sms))
+    return cudaLaunchKernelEx(&cfg, k_conv3d_smem<CIN, COUT>, nx, ny, nz, x, w, o, pdl ? 1 : 0);
+  cfg.gridDim = dim3((unsigned)(ntiles / nz * ((nz + 1) / 2)));
+  cfg.blockDim = dim3(ConvSmem2<CIN, COUT>::THREADS);
+  cfg.dynamicSmemBytes = ConvSmem2<CIN, COUT>::BYTES;
+  if constexpr (CIN == 16 && COUT == 32)
+    if (pack)
+      return cudaLaunchKernelEx(&cfg, k_conv3d_smem2<CIN, COUT, true>, nx, ny, nz, x, *pack, w, o, pdl ? 1 : 0);
+  return cudaLaunchKernelEx(&cfg, k_conv3d_smem2<CIN, COUT, false>, nx, ny, nz, x, PackIn{}, w, o, pdl ? 1 : 0);
 }
 
-// which convolution kernel launch_cnn_conv3d uses (LEXGB_CNN_AUTO: tcgen05 where the grid fits its
-// 8 x 16 tiles and has at least kConvTcMinPoints points, else mma.sync); process-wide, set by
-// lexgb_cnn_set_kernel
+// which convolution kernel conv3d uses (LEXGB_CNN_AUTO: tcgen05 where the grid fits its 8 x 16 tiles and
+// has at least kConvTcMinPoints points, else mma.sync); process-wide, set by lexgb_cnn_set_kernel.  The
+// line is where the two sum in different orders for a caller's results: below it tcgen05 is now the
+// faster one as well (the four layers at 64x64x32: 55 us against 103), but its last
+// bits, rounded to BF16 between layers, are other ones.
 int g_conv_kernel = LEXGB_CNN_AUTO;
-constexpr long long kConvTcMinPoints = 1ll << 18;   // below: too few tiles for the tcgen05 pipeline
+constexpr long long kConvTcMinPoints = 1ll << 18;
 
-cudaError_t launch_cnn_conv3d(int nx, int ny, int nz, int cin, int cout, const void* x, const void* w,
-                              const float* bias, float* pre, void* ybf, float* yf, int gelu, int creal,
-                              cudaStream_t st, bool pdl) {
+static cudaError_t conv3d(int nx, int ny, int nz, int cin, int cout, const void* x, const void* w,
+                          const ConvEpilogue& o, cudaStream_t st, bool pdl) {
   const bool big = (long long)nx * ny * nz >= kConvTcMinPoints;
-  if (conv_tc_fits(nx, ny, nz, cin, cout, x, pre, ybf, yf) &&
+  if (conv_tc_fits(nx, ny, nz, cin, cout, x, o) &&
       (g_conv_kernel == LEXGB_CNN_TCGEN05 || (g_conv_kernel == LEXGB_CNN_AUTO && big)))
-    return launch_conv_tc(nx, ny, nz, cin, cout, x, w, bias, pre, ybf, yf, gelu, creal, st, pdl);
+    return launch_conv_tc(nx, ny, nz, cin, cout, x, w, o, st, pdl);
   if (g_conv_kernel == LEXGB_CNN_TCGEN05) return cudaErrorInvalidValue;
   if (!(cin == 16 || cin == 32) || !(cout == 8 || cout == 16 || cout == 32) || nx % 16) return cudaErrorInvalidValue;
   const __nv_bfloat16* xb = (const __nv_bfloat16*)x;
   const __nv_bfloat16* wb = (const __nv_bfloat16*)w;
-  __nv_bfloat16* yb = (__nv_bfloat16*)ybf;
-#define LEXGB_CONV(CI, CO) launch_conv_smem<CI, CO>(nx, ny, nz, xb, wb, bias, pre, yb, yf, gelu, creal, st, pdl)
+#define LEXGB_CONV(CI, CO) launch_conv_smem<CI, CO>(nx, ny, nz, xb, wb, o, st, pdl)
   if (cin == 16) return cout == 8 ? LEXGB_CONV(16, 8) : cout == 16 ? LEXGB_CONV(16, 16) : LEXGB_CONV(16, 32);
   return cout == 8 ? LEXGB_CONV(32, 8) : cout == 16 ? LEXGB_CONV(32, 16) : LEXGB_CONV(32, 32);
 #undef LEXGB_CONV
 }
 
-cudaError_t conv_prepare() {
-  int cap;
-  cudaError_t e;
-  if ((e = conv_tc_prepare()) != cudaSuccess) return e;
-  if ((e = conv_grid<16, 8>(&cap)) != cudaSuccess) return e;
-  if ((e = conv_grid<16, 16>(&cap)) != cudaSuccess) return e;
-  if ((e = conv_grid<16, 32>(&cap)) != cudaSuccess) return e;
-  if ((e = conv_grid<32, 8>(&cap)) != cudaSuccess) return e;
-  if ((e = conv_grid<32, 16>(&cap)) != cudaSuccess) return e;
-  return conv_grid<32, 32>(&cap);
+cudaError_t launch_cnn_conv3d(int nx, int ny, int nz, int cin, int cout, const void* x, const void* w,
+                              const float* bias, float* pre, void* ybf, float* yf, int gelu, int creal,
+                              cudaStream_t st, bool pdl) {
+  ConvEpilogue o;
+  o.bias = bias;
+  o.pre = pre;
+  o.ybf = ybf;
+  o.yf = yf;
+  o.gelu = gelu;
+  o.creal = creal;
+  return conv3d(nx, ny, nz, cin, cout, x, w, o, st, pdl);
 }
 
-cudaError_t launch_sgs_pack(int nx, int ny, int nz, const float* T, const float* u, const float* v, const float* w,
-                            const float* q, float theta_ref, const float* lo, const float* rin, void* x16,
-                            cudaStream_t st) {
-  const long long n = (long long)nx * ny * nz;
-  k_sgs_pack<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(nx, ny, nz, T, u, v, w, q, theta_ref, lo, rin,
-                                                          (uint4*)x16);
+// dw[27][cout][cin] += sum_p g[p][co] x[p+off][ci] on the kernel that fits
+static cudaError_t weight_grad(int nx, int ny, int nz, int cin, int cout, int gstride, const void* x, const void* g,
+                               float* dw, cudaStream_t st) {
+  if (g_conv_kernel != LEXGB_CNN_MMA && conv_dw_tc_fits(nx, ny, nz, cin, cout, gstride, x, g, dw))
+    return launch_conv_dw_tc(nx, ny, nz, cin, cout, gstride, x, g, dw, st);
+  if (g_conv_kernel == LEXGB_CNN_TCGEN05) return cudaErrorInvalidValue;
+  const long long npts = (long long)nx * ny * nz;
+  const dim3 grid((unsigned)((npts + SLAB - 1) / SLAB), 27);
+  const size_t smem = (size_t)SLAB * (cin + cout) * sizeof(float);
+  k_conv3d_dw<<<grid, 256, smem, st>>>(nx, ny, nz, cin, cout, gstride, (const __nv_bfloat16*)x,
+                                       (const __nv_bfloat16*)g, dw);
   return cudaGetLastError();
+}
+
+cudaError_t conv_prepare() {
+  int cap, sms;
+  cudaError_t e;
+  if ((e = conv_tc_prepare()) != cudaSuccess) return e;
+  if ((e = conv_grid<16, 8>(&cap, &sms)) != cudaSuccess) return e;
+  if ((e = conv_grid<16, 16>(&cap, &sms)) != cudaSuccess) return e;
+  if ((e = conv_grid<16, 32>(&cap, &sms)) != cudaSuccess) return e;
+  if ((e = conv_grid<32, 8>(&cap, &sms)) != cudaSuccess) return e;
+  if ((e = conv_grid<32, 16>(&cap, &sms)) != cudaSuccess) return e;
+  return conv_grid<32, 32>(&cap, &sms);
+}
+
+cudaError_t launch_sgs_input(int nx, int ny, int nz, const float* T, const float* u, const float* v, const float* w,
+                             const float* q, float theta_ref, const float* lo, const float* rin, void* x16,
+                             const void* w0, const float* b0, void* out, cudaStream_t st, bool pdl) {
+  PackIn in;
+  in.T = T;
+  in.u = u;
+  in.v = v;
+  in.w = w;
+  in.q = q;
+  in.theta_ref = theta_ref;
+  in.lo = lo;
+  in.rin = rin;
+  ConvEpilogue o;
+  o.bias = b0;
+  o.ybf = out;
+  o.gelu = 1;
+  o.creal = 32;
+  int cap = 0, sms = 0;
+  cudaError_t e = conv_grid<16, 32>(&cap, &sms);
+  if (e != cudaSuccess) return e;
+  const long long n = (long long)nx * ny * nz;
+  if (nx % 16 == 0 && n < kConvTcMinPoints && g_conv_kernel != LEXGB_CNN_TCGEN05 && conv_pairs(nx, ny, nz, sms))
+    return launch_conv_smem<16, 32>(nx, ny, nz, (const __nv_bfloat16*)x16, (const __nv_bfloat16*)w0, o, st, pdl, &in);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((n + 255) / 256));
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl ? 1 : 0;
+  e = cudaLaunchKernelEx(&cfg, k_sgs_pack, nx, ny, nz, in, (uint4*)x16);
+  return e != cudaSuccess ? e : conv3d(nx, ny, nz, 16, 32, x16, w0, o, st, pdl);
 }
 
 cudaError_t launch_sgs_unpack(int nx, int ny, int nz, const float* corr, const float* rout, float* T, float* u,
@@ -639,20 +1015,120 @@ extern "C" int lexgb_cnn_conv3d_dw(int nx, int ny, int nz, int cin, int cout, in
     return cnn_arg("lexgb_cnn_conv3d_dw: bad argument (cin, cout <= 32, cout divides 256, gstride >= cout)");
   const long long npts = (long long)nx * ny * nz;
   cudaStream_t st = (cudaStream_t)stream;
-  if (g_conv_kernel != LEXGB_CNN_MMA && conv_dw_tc_fits(nx, ny, nz, cin, cout, gstride, x, g, dw)) {
-    const cudaError_t e = launch_conv_dw_tc(nx, ny, nz, cin, cout, gstride, x, g, dw, st);
-    if (e != cudaSuccess) return cnn_status(e, "lexgb_cnn_conv3d_dw (tcgen05)");
-  } else if (g_conv_kernel == LEXGB_CNN_TCGEN05) {
+  if (g_conv_kernel == LEXGB_CNN_TCGEN05 && !conv_dw_tc_fits(nx, ny, nz, cin, cout, gstride, x, g, dw))
     return cnn_arg("lexgb_cnn_conv3d_dw: the tcgen05 kernel needs cin 16 or 32, gstride 16 or 32, cout <= gstride "
                    "and 16-byte aligned x and g");
-  } else {
-    dim3 grid((unsigned)((npts + SLAB - 1) / SLAB), 27);
-    const size_t smem = (size_t)SLAB * (cin + cout) * sizeof(float);
-    k_conv3d_dw<<<grid, 256, smem, st>>>(nx, ny, nz, cin, cout, gstride, (const __nv_bfloat16*)x,
-                                         (const __nv_bfloat16*)g, dw);
-  }
+  const cudaError_t e = weight_grad(nx, ny, nz, cin, cout, gstride, x, g, dw, st);
+  if (e != cudaSuccess) return cnn_status(e, "lexgb_cnn_conv3d_dw");
   if (db) k_bias_grad<<<256, 256, 0, st>>>(npts, cout, gstride, (const __nv_bfloat16*)g, db);
   return cnn_status(cudaGetLastError(), "lexgb_cnn_conv3d_dw");
+}
+
+// ------------------------------------------------------------------------------------------------
+// the network's training pass
+// ------------------------------------------------------------------------------------------------
+namespace {
+constexpr int NET_CIN[4] = {16, 32, 32, 32}, NET_COUT[4] = {32, 32, 32, 8};
+constexpr int NET_REAL = 5;
+
+unsigned pad_blocks(long long n) {
+  const long long b = (n + 255) / 256;
+  return (unsigned)(b < 1216 ? b : 1216);   // 8 blocks per SM: few additions to db
+}
+bool net_args(int nx, int ny, int nz, const void* const* p, int np) {
+  if (nx <= 0 || ny <= 0 || nz <= 0 || nx % 16) return false;
+  for (int i = 0; i < np; ++i)
+    if (!p[i]) return false;
+  return true;
+}
+}  // namespace
+
+extern "C" int lexgb_cnn_net_forward(int nx, int ny, int nz, const float* x, const void* const w[4],
+                                     const float* const b[4], void* const act[4], float* const pre[3], float* out,
+                                     void* stream) {
+  using namespace lexgb;
+  if (!w || !b || !act || !pre || !out) return cnn_arg("lexgb_cnn_net_forward: null argument");
+  const void* all[15] = {w[0], w[1], w[2], w[3], b[0], b[1], b[2], b[3], act[0], act[1], act[2], act[3], pre[0], pre[1], pre[2]};
+  if (!net_args(nx, ny, nz, all, 15))
+    return cnn_arg("lexgb_cnn_net_forward: null argument, or nx not a positive multiple of 16");
+  cudaStream_t st = (cudaStream_t)stream;
+  const long long n = (long long)nx * ny * nz;
+  if (x) {
+    k_pad5<<<pad_blocks(n), 256, 0, st>>>(n, x, (uint4*)act[0], nullptr);
+    if (cudaError_t e = cudaGetLastError()) return cnn_status(e, "lexgb_cnn_net_forward");
+  }
+  for (int l = 0; l < 4; ++l) {
+    const bool last = l == 3;
+    ConvEpilogue o;
+    o.bias = b[l];
+    o.pre = last ? nullptr : pre[l];
+    o.ybf = last ? nullptr : act[l + 1];
+    o.yf = last ? out : nullptr;
+    o.gelu = !last;
+    o.creal = last ? NET_REAL : NET_COUT[l];
+    o.compact = last;
+    // each layer stages its weights, which no kernel of this call writes, while the previous one drains
+    const cudaError_t e = conv3d(nx, ny, nz, NET_CIN[l], NET_COUT[l], act[l], w[l], o, st, true);
+    if (e != cudaSuccess) return cnn_status(e, "lexgb_cnn_net_forward");
+  }
+  return LEXGB_OK;
+}
+
+extern "C" int lexgb_cnn_net_backward(int nx, int ny, int nz, const float* gout, const void* const w[4],
+                                      const void* const act[4], const float* const pre[3], void* work, float* grads,
+                                      float* dx, void* stream) {
+  using namespace lexgb;
+  if (!gout || !w || !act || !pre || !work || !grads || !dx) return cnn_arg("lexgb_cnn_net_backward: null argument");
+  const void* all[11] = {w[0], w[1], w[2], w[3], act[0], act[1], act[2], act[3], pre[0], pre[1], pre[2]};
+  if (!net_args(nx, ny, nz, all, 11))
+    return cnn_arg("lexgb_cnn_net_backward: null argument, or nx not a positive multiple of 16");
+  cudaStream_t st = (cudaStream_t)stream;
+  const long long n = (long long)nx * ny * nz;
+  // work: two gradients of 32 channels (the first also holds the 16 channels at the output), then the
+  // mirrored weights; grads: dw of the four layers, then db
+  __nv_bfloat16* const g[2] = {(__nv_bfloat16*)work, (__nv_bfloat16*)work + n * 32};
+  MirrorArgs m;
+  __nv_bfloat16* wm = g[1] + n * 32;
+  float *dw[4], *db[4], *q = grads;
+  int end = 0;
+  for (int l = 0; l < 4; ++l) {
+    m.w[l] = (const __nv_bfloat16*)w[l];
+    m.cin[l] = NET_CIN[l];
+    m.cout[l] = NET_COUT[l];
+    m.g[l] = l == 3 ? 16 : 32;
+    m.out[l] = wm + end;
+    m.end[l] = end += 27 * m.cin[l] * m.g[l];
+    dw[l] = q;
+    q += 27 * NET_CIN[l] * NET_COUT[l];
+  }
+  for (int l = 0; l < 4; ++l) {
+    db[l] = q;
+    q += NET_COUT[l];
+  }
+  cudaError_t e = cudaMemsetAsync(grads, 0, (size_t)(q - grads) * sizeof(float), st);
+  if (e == cudaSuccess) {
+    k_mirror<<<(end + 255) / 256, 256, 0, st>>>(m);
+    k_pad5<<<pad_blocks(n), 256, 0, st>>>(n, gout, (uint4*)g[0], db[3]);
+    e = cudaGetLastError();
+  }
+  for (int l = 3; l >= 0 && e == cudaSuccess; --l) {
+    const __nv_bfloat16* in = g[(3 - l) & 1];
+    e = weight_grad(nx, ny, nz, NET_CIN[l], NET_COUT[l], m.g[l], act[l], in, dw[l], st);
+    if (e != cudaSuccess) break;
+    // the input gradient, times GELU' of the layer below, as that layer's output gradient
+    ConvEpilogue o;
+    o.creal = l ? NET_CIN[l] : NET_REAL;
+    o.compact = l == 0;
+    if (l) {
+      o.gpre = pre[l - 1];
+      o.ybf = g[(4 - l) & 1];
+      o.db = db[l - 1];
+    } else {
+      o.yf = dx;
+    }
+    e = conv3d(nx, ny, nz, m.g[l], NET_CIN[l], in, m.out[l], o, st, true);
+  }
+  return cnn_status(e, "lexgb_cnn_net_backward");
 }
 
 extern "C" int lexgb_cnn_adam(long long n, float* w, const float* gw, float* m, float* v, void* w_bf16, float lr,

@@ -9,22 +9,31 @@
 // input tile is read by the tensor cores 9 x Cin/16 times per plane instead of 27 x Cin/16.
 // A block owns a column of 8 (x) x 16 (y) points and marches up a chunk of levels, with its
 // warps specialised:
-//   warp 4 (producer)  loads each input plane the chunk needs (10 x 18 points with the one-point
+//   the producer warp  loads each input plane the chunk needs (10 x 18 points with the one-point
 //                      halo, zero outside the grid by the tensor map's out-of-bounds fill) by TMA
 //                      (cp.async.bulk.tensor, one box per 8-channel group) into a ring of plane
 //                      slots; a slot's full barrier completes on the bytes' arrival;
-//   warp 5 (MMA)       for plane p issues the 9 x Cin/16 MMAs (M = 128, N = 3 NP, K = 16, BF16
+//   the MMA warp       for plane p issues the 9 x Cin/16 MMAs (M = 128, N = 3 NP, K = 16, BF16
 //                      in, FP32 accumulate) into the columns of output levels p+1, p, p-1: the
 //                      tensor memory is a ring of Q level slots of NP columns in descending level
 //                      order, so the three are adjacent (where they wrap round the ring, the MMA
-//                      is split in two; never in a chunk of at most Q - 5 levels); it frees the
-//                      plane's slot and marks level p-1 summed;
-//   warps 0-3          (the four tensor-memory lane quarters) zero the ring first (the windows of
+//                      is split in two; rows of levels outside the chunk are left out of N); it
+//                      frees the plane's slot and marks level p-1 summed;
+//   the epilogue warps (one per tensor-memory lane quarter and 16 channels) zero the ring first (the windows of
 //                      neighbouring planes overlap, so every MMA accumulates), then for each level
 //                      wait for it, read their 32 rows (tcgen05.ld), zero the level slot again if
 //                      a later level of the chunk uses it, hand it back to the MMA warp and apply
-//                      the epilogue of k_conv3d_smem (bias, FP32 pre-activation, GELU, padding
-//                      channels zero, BF16 / FP32 output).
+//                      the epilogue (ConvEpilogue).  A lane's tensor-memory row is one point's
+//                      channels; stored from there, a store instruction would touch 32 lines with
+//                      16 bytes each, so the rows go through shared memory first and each
+//                      instruction moves 64 consecutive bytes of FP32 of 8 points.
+// What bounds it at 128x128x64 (two blocks per SM, 256 blocks of 32 levels): taken apart by leaving
+// one part out of a copy, the epilogue and the MMAs of a plane each took 66 us for 32 -> 32 channels
+// when four warps stored whole rows, together 95 us; loads do not matter.  The MMAs (9 Cin/16 of
+// 128 x 96 x 16 a plane) are bound by reading A: a core matrix (8 points, 128 bytes) starts off a
+// 128-byte boundary for every shift, two shared-memory passes instead of one.  Eight epilogue warps
+// of 16 channels: 78 us (82 with the FP32 pre-activation; 120 and 182 with direct 16-byte stores and
+// chunks of 5 levels).
 // Every wait is bounded: one that gives up counts a timeout in g_tc_timeouts and sets the block's
 // abort flag, which ends the other roles' waits; the block then waits (bounded) for the MMAs it
 // issued and the copies in flight, frees its tensor memory and returns.
@@ -61,7 +70,7 @@ struct TcLayout {
   static constexpr int NP = COUT < 16 ? 16 : COUT;  // output channels of one level in N (16 or 32)
   static constexpr int N3 = 3 * NP;                 // N of the MMA: output levels p+1, p, p-1
   static constexpr int CG = CIN / 8;                // channel groups of 8 (16 bytes)
-  static constexpr int R = 4;                       // plane slots (each plane is read once)
+  static constexpr int R = CIN * COUT == 1024 ? 3 : 4;   // plane slots (each plane is read once; two blocks per SM)
   static constexpr int TMEM_COLS = 256;             // two blocks per SM
   static constexpr int Q = TMEM_COLS / NP;          // level slots of NP columns (8 or 16)
   static constexpr int W_BYTES = 9 * CG * N3 * 16;
@@ -71,13 +80,16 @@ struct TcLayout {
   static constexpr int A_SBO = TC_HX * 16;          // next row of the tile (8 points on)
   static constexpr int B_LBO = N3 * 16;             // next input-channel group
   static constexpr int B_SBO = 128;                 // next 8 rows of N
-  static constexpr int EPI = 4;                     // epilogue warps (one per tensor-memory lane quarter)
+  static constexpr int HC = COUT < 16 ? COUT : 16;  // output channels of an epilogue warp
+  static constexpr int EPI = 4 * (COUT / HC);       // epilogue warps: one per tensor-memory lane quarter and channel part
   static constexpr int THREADS = 32 * (EPI + 2);    // + the producer and the MMA warp
   static constexpr int NBAR = 2 * R + 2 * Q + 1;    // full[R], empty[R], summed[Q], freed[Q], done
-  static constexpr int BAR_BYTES = NBAR * 8 + 16;
+  static constexpr int BAR_BYTES = (NBAR * 8 + 16 + 15) / 16 * 16;   // + tensor-memory address, abort flag
   // + alignment slack, barriers, tensor-memory address, abort flag, bias; at least 80 KB, so that
   // no more blocks share an SM than its tensor memory holds
-  static constexpr size_t NEED = 128 + (size_t)W_BYTES + P_BYTES + BAR_BYTES + NP * 4;
+  static constexpr int SR = HC + 4;                 // staged epilogue row (floats): conflict-free 16-byte accesses
+  static constexpr int ST_OFF = (W_BYTES + P_BYTES + BAR_BYTES + 2 * NP * 4 + 15) / 16 * 16;   // bias, db sums before it
+  static constexpr size_t NEED = 128 + (size_t)ST_OFF + EPI * 32 * SR * 4;
   static constexpr size_t BYTES = NEED < 80 * 1024 ? 80 * 1024 : NEED;
 };
 
@@ -107,6 +119,15 @@ __device__ __forceinline__ void mma_bf16_tc(uint32_t tmem_d, uint64_t adesc, uin
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+}
+
+// One lane of the (converged) warp.  Inside `if (elect_one())` the compiler knows a single thread runs
+// and keeps the MMA descriptors in uniform registers; behind `lane == 0` each MMA moved its descriptors
+// there first, 107 cycles an MMA whatever its size.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+  return p != 0;
 }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -223,94 +244,79 @@ __device__ __forceinline__ void tmem_zero_cols(uint32_t taddr) {
   }
 }
 
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(TcLayout<CIN, COUT>::THREADS, 1)
-    k_conv3d_tc(const __grid_constant__ CUtensorMap xmap, int nx, int ny, int nz, int zc,
-                const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias, float* __restrict__ pre,
-                __nv_bfloat16* __restrict__ ybf, float* __restrict__ yf, int gelu, int creal, int early_weights) {
-  using L = TcLayout<CIN, COUT>;
-  constexpr int NP = L::NP, N3 = L::N3, CG = L::CG, R = L::R, Q = L::Q, EPI = L::EPI;
-  constexpr int H = EPI / 4, CW = NP / H;   // channel parts of a level; columns of one part
-  extern __shared__ unsigned char tc_raw[];
-  const uint32_t raw_s = smem_u32(tc_raw);
-  unsigned char* smem = tc_raw + ((128u - (raw_s & 127u)) & 127u);   // 128-byte aligned for TMA
-  const uint32_t w_s = smem_u32(smem), p_s = w_s + L::W_BYTES, bar_s = p_s + L::P_BYTES;
-  auto full = [&](int s) { return bar_s + 8u * s; };
-  auto empty = [&](int s) { return bar_s + 8u * (R + s); };
-  auto summed = [&](int q) { return bar_s + 8u * (2 * R + q); };       // a level slot's sums are complete
-  auto freed = [&](int q) { return bar_s + 8u * (2 * R + Q + q); };    // ... read (and zeroed if reused)
-  const uint32_t done = bar_s + 8u * (2 * R + 2 * Q);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::W_BYTES + L::P_BYTES + L::NBAR * 8);
-  volatile int* abort = reinterpret_cast<volatile int*>(tslot + 1);
-  float* bsm = reinterpret_cast<float*>(smem + L::W_BYTES + L::P_BYTES + L::BAR_BYTES);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+// Shared memory of a block's tile (addresses in the shared window where the tensor cores or TMA use them)
+struct TcSmem {
+  uint32_t w, p, bar;     // the layer's weights, plane slots, barriers
+  volatile int* abort;
+  float *bias, *db;       // NP floats each: the layer's biases, the block's sums for ConvEpilogue::db
+  float* stage;           // the epilogue warps' staged rows
+};
 
-  if (warp == EPI + 1) {  // tensor memory: Q level slots of NP columns
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
-                 "r"(L::TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  if (tid == 0) {
-    for (int s = 0; s < R; ++s) {
-      mbar_init(full(s), 1);
-      mbar_init(empty(s), 1);
+// Barriers of a tile: full[R], empty[R], summed[Q] (a level slot's sums are complete), freed[Q] (read,
+// and zeroed if reused), done
+template <class L>
+__device__ __forceinline__ void tc_barriers(uint32_t bar, int lane) {   // a warp
+  for (int b = lane; b < L::NBAR; b += 32)
+    mbar_init(bar + 8u * b, b >= 2 * L::R + L::Q && b < 2 * L::R + 2 * L::Q ? L::EPI : 1);
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+
+// weights Wsm[dy dx][cg][n][8] from w[tap][COUT][CIN]: row n = t NP + co holds the tap
+// (dz = t - 1, dy, dx) of output channel co (rows co >= COUT zero), so that one MMA on input
+// plane p adds to output levels p+1 (t = 0), p (t = 1) and p-1 (t = 2)
+template <class L, int CIN, int COUT>
+__device__ __forceinline__ void tc_stage_weights(uint32_t dst, const __nv_bfloat16* w, int warp, int lane) {
+  // a warp per tap, whose COUT x CIN weights lie together: 512 bytes of them an instruction (one that
+  // took a column of 16-byte pieces, as the rows lie in shared memory, spent 5 us on 55 KB)
+  constexpr int WARPS = L::THREADS / 32;
+  for (int tap = warp; tap < 27; tap += WARPS) {
+    const int t = tap / 9, yx = tap - 9 * t;
+#pragma unroll
+    for (int c0 = 0; c0 < L::NP * L::CG; c0 += 32) {
+      const int c = c0 + lane, co = c / L::CG, cg = c % L::CG;
+      const bool ok = co < COUT;
+      cp16(dst + (uint32_t)(((yx * L::CG + cg) * L::N3 + t * L::NP + co) * 16),
+           w + (ok ? tap * COUT * CIN + c * 8 : 0), ok);
     }
-    for (int q = 0; q < Q; ++q) {
-      mbar_init(summed(q), 1);
-      mbar_init(freed(q), EPI);
-    }
-    mbar_init(done, 1);
-    *abort = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  // weights Wsm[dy dx][cg][n][8] from w[tap][COUT][CIN]: row n = t NP + co holds the tap
-  // (dz = t - 1, dy, dx) of output channel co (rows co >= COUT zero), so that one MMA on input
-  // plane p adds to output levels p+1 (t = 0), p (t = 1) and p-1 (t = 2)
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (!early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
-  for (int e = tid; e < 9 * CG * N3; e += L::THREADS) {
-    const int n = e % N3, cg = (e / N3) % CG, yx = e / (N3 * CG);
-    const int t = n / NP, co = n % NP;
-    const bool ok = co < COUT;
-    const int tap = t * 9 + yx;
-    cp16(w_s + (uint32_t)e * 16u, w + ((long long)(tap * COUT + (ok ? co : 0)) * CIN + cg * 8), ok);
-  }
-  if (tid < NP) bsm[tid] = (bias && tid < COUT) ? bias[tid] : 0.f;
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tslot;
-  // epilogue warp w: lanes 32 (w % 4) .., channels CW (w / 4) .. of every level
+}
+
+// epilogue warps: zero this warp's lanes and channels of the level slots in use (the MMA windows of
+// neighbouring planes overlap, so they all accumulate)
+template <class L>
+__device__ __forceinline__ void tc_zero(uint32_t tmem, int warp, int levels) {
+  if (warp >= L::EPI) return;
+  const uint32_t at = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((warp >> 2) * 16);
+  for (int q = L::Q - min(levels, L::Q); q < L::Q; ++q) tmem_zero_cols<16>(at + (uint32_t)(q * L::NP));
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// One tile of 8 x 16 points and the levels z0 .. z1-1: the roles of the block's warps, from
+// initialised barriers, staged weights and zeroed level slots.
+template <class L, int CIN, int COUT>
+__device__ __forceinline__ void tc_tile(const CUtensorMap& xmap, int nx, int ny, int x0, int y0, int z0, int z1,
+                                        const TcSmem& m, uint32_t tmem, const ConvEpilogue& o) {
+  constexpr int NP = L::NP, N3 = L::N3, CG = L::CG, R = L::R, Q = L::Q, EPI = L::EPI;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  volatile int* const abort = m.abort;
+  auto full = [&](int s) { return m.bar + 8u * s; };
+  auto empty = [&](int s) { return m.bar + 8u * (R + s); };
+  auto summed = [&](int q) { return m.bar + 8u * (2 * R + q); };
+  auto freed = [&](int q) { return m.bar + 8u * (2 * R + Q + q); };
+  const uint32_t done = m.bar + 8u * (2 * R + 2 * Q);
+  // epilogue warp w: lanes 32 (w % 4) .., columns part .. part + CW - 1 of every level
+  constexpr int CW = 16;
   const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
   const int part = (warp >> 2) * CW;
-  // the MMA windows of neighbouring planes overlap, so they all accumulate: zero the slots first
-  if (warp < EPI) {
-    for (int q = 0; q < Q; ++q) tmem_zero_cols<CW>(tmem + lanes + (uint32_t)(q * NP + part));
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-  }
-  asm volatile("cp.async.wait_all;" ::: "memory");
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // weights -> the tensor cores
-  if (early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");   // the input is ready
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-
-  const int tiles_x = nx / TC_TX, tiles_y = ny / TC_TY;
-  const int tx = blockIdx.x % tiles_x, ty = (blockIdx.x / tiles_x) % tiles_y, ch = blockIdx.x / (tiles_x * tiles_y);
-  const int x0 = tx * TC_TX, y0 = ty * TC_TY, z0 = ch * zc, z1 = min(z0 + zc, nz);
   const int p0 = z0 - 1;   // first plane of the chunk; plane p uses slot (p - p0) % R, fill (p - p0) / R
-  // Output level z (z0 - 2 .. z1 + 1; the four outside z0 .. z1 - 1 are scratch that the planes at
-  // the chunk's ends add to) lives in level slot Q - 1 - (z - z0 + 2) mod Q, its (z - z0 + 2) / Q-th
-  // use: the slots of levels p+1, p, p-1 follow one another except where they wrap round (never in
-  // a chunk of at most Q - 5 levels).
-  const int zb = z0 - 2;
-  auto lslot = [&](int z) { return Q - 1 - (z - zb) % Q; };
-  auto luse = [&](int z) { return (z - zb) / Q; };
+  // Output level z of the chunk lives in level slot Q - 1 - (z - z0) mod Q, its (z - z0) / Q-th use:
+  // the slots of levels p+1, p, p-1 follow one another except where they wrap round
+  auto lslot = [&](int z) { return Q - 1 - (z - z0) % Q; };
+  auto luse = [&](int z) { return (z - z0) / Q; };
 
   if (warp == EPI) {
     // ---------------- producer: planes z0-1 .. z1 ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       int p = p0;
       for (; p <= z1; ++p) {
         const int s = (p - p0) % R, k = (p - p0) / R;
@@ -321,63 +327,82 @@ __global__ void __launch_bounds__(TcLayout<CIN, COUT>::THREADS, 1)
         }
         mbar_expect_tx(full(s), CG * TC_BOX_BYTES);
         for (int cg = 0; cg < CG; ++cg)
-          tma_load_4d(p_s + s * L::PLANE_BYTES + cg * TC_GROUP_BYTES, &xmap, cg * 8, x0 - 1, y0 - 1, p, full(s));
+          tma_load_4d(m.p + s * L::PLANE_BYTES + cg * TC_GROUP_BYTES, &xmap, cg * 8, x0 - 1, y0 - 1, p, full(s));
       }
       // the copies this thread issued have landed before the block's memory goes (bounded)
       for (int q = p - 1; q >= p0 && q >= p - R; --q) mbar_wait_long(full((q - p0) % R), ((q - p0) / R) & 1, nullptr);
     }
   } else if (warp == EPI + 1) {
     // ---------------- MMA issuer: one plane at a time ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       // descriptors: the start address is the low field (16-byte units), so an operand at a fixed
       // offset from a base is the base's descriptor plus the offset / 16
-      const uint64_t b0 = smem_desc(w_s, L::B_LBO, L::B_SBO);
+      const uint64_t b0 = smem_desc(m.w, L::B_LBO, L::B_SBO);
       bool ok = true;
+      int s = 0, k = 0;   // plane slot and fill
       for (int p = p0; p <= z1 && ok; ++p) {
-        const int s = (p - p0) % R, k = (p - p0) / R;
         ok = mbar_wait(full(s), k & 1, abort);
         // level p+1 is new in its slot: the level that used the slot before has been read and zeroed
-        if (ok && luse(p + 1) > 0) ok = mbar_wait(freed(lslot(p + 1)), (luse(p + 1) - 1) & 1, abort);
+        if (ok && p + 1 < z1 && luse(p + 1) > 0) ok = mbar_wait(freed(lslot(p + 1)), (luse(p + 1) - 1) & 1, abort);
         if (!ok) {
           atomicAdd(&g_tc_timeouts, 1u);
           *abort = 1;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int q0 = lslot(p + 1);   // slots q0, q0 + 1, q0 + 2 (mod Q) <- t = 0, 1, 2
-        // the rows t < split go to columns q0 NP.., the rest to column 0 (the window wraps)
-        const int split = q0 + 3 <= Q ? 3 : Q - q0;
+        // the rows t = 0, 1, 2 of N add to levels p+1, p, p-1; those of the chunk are t = ta .. tb-1
+        const int ta = max(0, p + 2 - z1), tb = min(3, p + 2 - z0);
+        const int q0 = lslot(p + 1 - ta);           // level p+1-ta's slot; the next rows' slots follow
+        const int n1 = min(tb - ta, Q - q0);        // rows before the window wraps to column 0
+        const int n2 = tb - ta - n1;
         const uint32_t c_hi = tmem + (uint32_t)(q0 * NP), c_lo = tmem;
-        const uint64_t a0 = smem_desc(p_s + s * L::PLANE_BYTES, L::A_LBO, L::A_SBO);
+        const uint32_t id1 = tc_idesc(128, n1 * NP), id2 = tc_idesc(128, n2 * NP);
+        const uint64_t a0 = smem_desc(m.p + s * L::PLANE_BYTES, L::A_LBO, L::A_SBO);
+        const uint64_t b1 = b0 + (uint64_t)((ta * NP * 16) >> 4), b2 = b1 + (uint64_t)((n1 * NP * 16) >> 4);
+        auto taps = [&](uint32_t col, uint64_t bd, uint32_t id) {
 #pragma unroll
-        for (int dy = 0; dy < 3; ++dy)
+          for (int dy = 0; dy < 3; ++dy)
 #pragma unroll
-          for (int dx = 0; dx < 3; ++dx)
+            for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
-            for (int ks = 0; ks < CIN / 16; ++ks) {
-              const uint64_t ad = a0 + (uint64_t)((2 * ks * TC_GROUP_BYTES + (dy * TC_HX + dx) * 16) >> 4);
-              const uint64_t bd = b0 + (uint64_t)((((dy * 3 + dx) * CG + 2 * ks) * N3 * 16) >> 4);
-              if (split == 3) {
-                mma_bf16_tc(c_hi, ad, bd, tc_idesc(128, N3), 1u);
-              } else if (split == 2) {
-                mma_bf16_tc(c_hi, ad, bd, tc_idesc(128, 2 * NP), 1u);
-                mma_bf16_tc(c_lo, ad, bd + (uint64_t)((2 * NP * 16) >> 4), tc_idesc(128, NP), 1u);
-              } else {
-                mma_bf16_tc(c_hi, ad, bd, tc_idesc(128, NP), 1u);
-                mma_bf16_tc(c_lo, ad, bd + (uint64_t)((NP * 16) >> 4), tc_idesc(128, 2 * NP), 1u);
-              }
-            }
+              for (int ks = 0; ks < CIN / 16; ++ks)
+                mma_bf16_tc(col, a0 + (uint64_t)((2 * ks * TC_GROUP_BYTES + (dy * TC_HX + dx) * 16) >> 4),
+                            bd + (uint64_t)((((dy * 3 + dx) * CG + 2 * ks) * N3 * 16) >> 4), id, 1u);
+        };
+        taps(c_hi, b1, id1);
+        if (n2 > 0) taps(c_lo, b2, id2);
         mma_commit(empty(s));               // plane p is not read again
-        mma_commit(summed(lslot(p - 1)));   // level p-1 has all three of its planes
+        if (p > z0) mma_commit(summed(lslot(p - 1)));   // level p-1 has all three of its planes
+        if (++s == R) {
+          s = 0;
+          ++k;
+        }
       }
       mma_commit(done);
       mbar_wait_long(done, 0, nullptr);   // the MMAs are complete before the tensor memory goes
     }
-  } else {
+  } else if (warp < EPI) {
     // ---------------- epilogue: warps 0 .. EPI-1 ----------------
-    const int r = 32 * (warp & 3) + lane;   // row r <-> point (x0 + r % 8, y0 + r / 8)
-    for (int z = zb; z < z1; ++z) {
+    // row r of the tile <-> point (x0 + r % 8, y0 + r / 8); stores: pass i of a level takes points
+    // i PPP + lane / CPP of the warp's 32, a lane 4 channels from ch
+    constexpr int HC = L::HC, CPP = HC / 4, PPP = 32 / CPP;
+    const int c4 = 4 * (lane % CPP), ch = part + c4, pl = lane / CPP;
+    float* const st = m.stage + warp * 32 * L::SR;
+    const float4 b4 = *reinterpret_cast<const float4*>(m.bias + ch);
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    // the lane's point of pass i is at + i step (PPP points are PPP / 8 rows of the tile)
+    const int r0 = 32 * (warp & 3) + pl;
+    const long long at0 = (long long)(y0 + r0 / TC_TX) * nx + x0 + r0 % TC_TX, step = (long long)(PPP / TC_TX) * nx;
+    const bool masked = ch + 3 >= o.creal;
+    for (int z = z0; z < z1; ++z) {
       const int q = lslot(z);
+      const long long at = (long long)z * ny * nx + at0;
+      float4 gp[CPP];
+      if (o.gpre) {   // in flight while the level is summed
+#pragma unroll
+        for (int i = 0; i < CPP; ++i)
+          gp[i] = __ldg(reinterpret_cast<const float4*>(o.gpre + (at + i * step) * COUT + ch));
+      }
       if (!__all_sync(0xffffffffu, mbar_wait(summed(q), luse(z) & 1, abort))) {   // warp-uniform
         if (lane == 0) {
           atomicAdd(&g_tc_timeouts, 1u);
@@ -387,60 +412,159 @@ __global__ void __launch_bounds__(TcLayout<CIN, COUT>::THREADS, 1)
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       float v[CW];
-      const bool real = z >= z0;
       const uint32_t cols = tmem + lanes + (uint32_t)(q * NP + part);
-      if (real) {
-        tmem_load_cols<CW>(cols, v);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      }
-      if (z + Q <= z1 + 1) {   // the slot's next level is in this chunk: zero it for that level
+      tmem_load_cols<CW>(cols, v);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if (z + Q < z1) {   // the slot's next level is in this chunk: zero it for that level
         tmem_zero_cols<CW>(cols);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(freed(q));
-      if (!real || part >= COUT) continue;
-      // the point's channels part .. part + CW - 1 (those below COUT) as 16-byte stores
-      const long long p = ((long long)z * ny + y0 + r / TC_TX) * nx + x0 + r % TC_TX;
-      constexpr int CN = CW < COUT ? CW : COUT;   // channels of this part below COUT (COUT % CW == 0 or COUT < CW)
 #pragma unroll
-      for (int c = 0; c < CN; ++c) v[c] += bsm[part + c];
-      if (pre) {
+      for (int c = 0; c < HC; c += 4)
+        *reinterpret_cast<float4*>(st + lane * L::SR + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+      __syncwarp();
+      float4 a[CPP];
 #pragma unroll
-        for (int c = 0; c < CN; c += 4)
-          *reinterpret_cast<float4*>(pre + p * COUT + part + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+      for (int i = 0; i < CPP; ++i) {
+        a[i] = *reinterpret_cast<const float4*>(st + (i * PPP + pl) * L::SR + c4);
+        a[i] = make_float4(a[i].x + b4.x, a[i].y + b4.y, a[i].z + b4.z, a[i].w + b4.w);
       }
+      __syncwarp();   // the staged rows are read before the next level's replace them
+      if (o.pre) {
 #pragma unroll
-      for (int c = 0; c < CN; ++c) {
-        const float t = gelu ? gelu_fast(v[c]) : v[c];
-        v[c] = part + c < creal ? t : 0.f;
+        for (int i = 0; i < CPP; ++i) *reinterpret_cast<float4*>(o.pre + (at + i * step) * COUT + ch) = a[i];
       }
-      if (ybf) {
+      if (o.gelu) {
 #pragma unroll
-        for (int c = 0; c < CN; c += 8) {
-          uint4 qq;
-          __nv_bfloat162 h0 = __floats2bfloat162_rn(v[c], v[c + 1]);
-          __nv_bfloat162 h1 = __floats2bfloat162_rn(v[c + 2], v[c + 3]);
-          __nv_bfloat162 h2 = __floats2bfloat162_rn(v[c + 4], v[c + 5]);
-          __nv_bfloat162 h3 = __floats2bfloat162_rn(v[c + 6], v[c + 7]);
-          qq.x = *reinterpret_cast<uint32_t*>(&h0);
-          qq.y = *reinterpret_cast<uint32_t*>(&h1);
-          qq.z = *reinterpret_cast<uint32_t*>(&h2);
-          qq.w = *reinterpret_cast<uint32_t*>(&h3);
-          *reinterpret_cast<uint4*>(ybf + p * COUT + part + c) = qq;
+        for (int i = 0; i < CPP; ++i)
+          a[i] = make_float4(gelu_fast(a[i].x), gelu_fast(a[i].y), gelu_fast(a[i].z), gelu_fast(a[i].w));
+      }
+      if (o.gpre) {
+#pragma unroll
+        for (int i = 0; i < CPP; ++i)
+          a[i] = make_float4(a[i].x * gelu_tanh_grad(gp[i].x), a[i].y * gelu_tanh_grad(gp[i].y),
+                             a[i].z * gelu_tanh_grad(gp[i].z), a[i].w * gelu_tanh_grad(gp[i].w));
+      }
+      if (masked) {
+#pragma unroll
+        for (int i = 0; i < CPP; ++i) {
+          if (ch >= o.creal) a[i].x = 0.f;
+          if (ch + 1 >= o.creal) a[i].y = 0.f;
+          if (ch + 2 >= o.creal) a[i].z = 0.f;
+          a[i].w = 0.f;
         }
       }
-      if (yf) {
+      if (o.ybf) {
+        __nv_bfloat16* const y = reinterpret_cast<__nv_bfloat16*>(o.ybf) + at * COUT + ch;
 #pragma unroll
-        for (int c = 0; c < CN; c += 4)
-          *reinterpret_cast<float4*>(yf + p * COUT + part + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+        for (int i = 0; i < CPP; ++i) {
+          const __nv_bfloat162 lo = __floats2bfloat162_rn(a[i].x, a[i].y), hi = __floats2bfloat162_rn(a[i].z, a[i].w);
+          uint2 qq;
+          qq.x = *reinterpret_cast<const uint32_t*>(&lo);
+          qq.y = *reinterpret_cast<const uint32_t*>(&hi);
+          *reinterpret_cast<uint2*>(y + i * step * COUT) = qq;
+          const float2 l = __bfloat1622float2(lo), h = __bfloat1622float2(hi);
+          sum = make_float4(sum.x + l.x, sum.y + l.y, sum.z + h.x, sum.w + h.y);
+        }
+      }
+      if (o.yf && !o.compact) {
+#pragma unroll
+        for (int i = 0; i < CPP; ++i) *reinterpret_cast<float4*>(o.yf + (at + i * step) * COUT + ch) = a[i];
+      } else if (o.yf) {
+#pragma unroll
+        for (int i = 0; i < CPP; ++i) {
+          float* const y = o.yf + (at + i * step) * o.creal + ch;
+          if (ch < o.creal) y[0] = a[i].x;
+          if (ch + 1 < o.creal) y[1] = a[i].y;
+          if (ch + 2 < o.creal) y[2] = a[i].z;
+          if (ch + 3 < o.creal) y[3] = a[i].w;
+        }
+      }
+    }
+    if (o.db) {   // lanes with the same channels, then the block's warps
+#pragma unroll
+      for (int m = CPP; m < 32; m *= 2) {
+        sum.x += __shfl_xor_sync(0xffffffffu, sum.x, m);
+        sum.y += __shfl_xor_sync(0xffffffffu, sum.y, m);
+        sum.z += __shfl_xor_sync(0xffffffffu, sum.z, m);
+        sum.w += __shfl_xor_sync(0xffffffffu, sum.w, m);
+      }
+      if (lane < CPP) {
+        atomicAdd(m.db + ch, sum.x);
+        atomicAdd(m.db + ch + 1, sum.y);
+        atomicAdd(m.db + ch + 2, sum.z);
+        atomicAdd(m.db + ch + 3, sum.w);
       }
     }
   }
+}
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(TcLayout<CIN, COUT>::THREADS, 2)
+    k_conv3d_tc(const __grid_constant__ CUtensorMap xmap, int nx, int ny, int nz, int zc,
+                const __nv_bfloat16* __restrict__ w, const ConvEpilogue o, int early_weights) {
+  using L = TcLayout<CIN, COUT>;
+  extern __shared__ unsigned char tc_raw[];
+  const uint32_t raw_s = smem_u32(tc_raw);
+  unsigned char* smem = tc_raw + ((128u - (raw_s & 127u)) & 127u);   // 128-byte aligned for TMA
+  TcSmem m;
+  m.w = smem_u32(smem);
+  m.p = m.w + L::W_BYTES;
+  m.bar = m.p + L::P_BYTES;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::W_BYTES + L::P_BYTES + L::NBAR * 8);
+  m.abort = reinterpret_cast<volatile int*>(tslot + 1);
+  m.bias = reinterpret_cast<float*>(smem + L::W_BYTES + L::P_BYTES + L::BAR_BYTES);
+  m.db = m.bias + L::NP;
+  m.stage = reinterpret_cast<float*>(smem + L::ST_OFF);
+  const int tid = threadIdx.x, warp = tid >> 5;
+
+  // the weights' copies leave first: they, the tensor memory and the barriers are the whole of a small
+  // launch's start
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (!early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
+  tc_stage_weights<L, CIN, COUT>(m.w, w, warp, tid & 31);
+  if (warp == L::EPI + 1) {  // tensor memory: Q level slots of NP columns
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
+                 "r"(L::TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (warp == 1) {
+    if ((tid & 31) == 0) *m.abort = 0;
+    tc_barriers<L>(m.bar, tid & 31);
+  }
+  if (tid < L::NP) {   // the bias lands with the weights
+    if (o.bias && tid < COUT)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(m.bias + tid)), "l"(o.bias + tid) : "memory");
+    else
+      m.bias[tid] = 0.f;
+    m.db[tid] = 0.f;
+  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == EPI + 1) {
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tslot;
+  tc_zero<L>(tmem, warp, zc);
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // weights -> the tensor cores
+  const int tiles_x = nx / TC_TX, tiles_y = ny / TC_TY;
+  const int tx = blockIdx.x % tiles_x, ty = (blockIdx.x / tiles_x) % tiles_y, ch = blockIdx.x / (tiles_x * tiles_y);
+  const int x0 = tx * TC_TX, y0 = ty * TC_TY, z0 = ch * zc, z1 = min(z0 + zc, nz);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  // the threads that read the previous kernel's output or write over what it read (all but the MMA
+  // warp's) wait for it themselves: the first plane's copy leaves as soon as it can
+  if (early_weights && warp != L::EPI + 1) asm volatile("griddepcontrol.wait;" ::: "memory");
+  tc_tile<L, CIN, COUT>(xmap, nx, ny, x0, y0, z0, z1, m, tmem, o);
+
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (o.db && tid < COUT) atomicAdd(o.db + tid, m.db[tid]);
+  if (warp == L::EPI + 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(L::TMEM_COLS) : "memory");
   }
@@ -643,27 +767,24 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 constexpr int TC_MAX_DEVICES = 64;
 
 template <int CIN, int COUT>
-cudaError_t tc_grid(int* cap) {
-  static int grid_cap[TC_MAX_DEVICES] = {};
+cudaError_t tc_setup(int* sms) {
+  static int count[TC_MAX_DEVICES] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= TC_MAX_DEVICES) return cudaErrorInvalidDevice;
-  if (!grid_cap[dev]) {
+  if (!count[dev]) {
     using L = TcLayout<CIN, COUT>;
     e = cudaFuncSetAttribute(k_conv3d_tc<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_conv3d_tc<CIN, COUT>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              (int)cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
-    int sms = 0, per = 0;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_conv3d_tc<CIN, COUT>, L::THREADS, L::BYTES)) !=
-        cudaSuccess)
-      return e;
-    grid_cap[dev] = sms * (per < 1 ? 1 : per);
+    int n = 0;
+    if ((e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    count[dev] = n;
   }
-  *cap = grid_cap[dev];
+  *sms = count[dev];
   return cudaSuccess;
 }
 
@@ -702,29 +823,38 @@ bool make_xmap(CUtensorMap* map, const void* x, int nx, int ny, int nz, int cin)
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int CIN, int COUT>
-cudaError_t launch_tc(int nx, int ny, int nz, const void* x, const __nv_bfloat16* w, const float* bias, float* pre,
-                      __nv_bfloat16* ybf, float* yf, int gelu, int creal, cudaStream_t st, bool pdl) {
-  int cap = 0;
-  cudaError_t e = tc_grid<CIN, COUT>(&cap);
-  if (e != cudaSuccess) return e;
-  CUtensorMap xmap;
-  if (!make_xmap(&xmap, x, nx, ny, nz, CIN)) return cudaErrorInvalidValue;
-  // level chunks of at least 4 levels: the count whose blocks fill their waves of resident blocks
-  // best (ties: fewer chunks, since every chunk stages the weights and two extra planes)
-  using L = TcLayout<CIN, COUT>;
-  const int tiles = (nx / TC_TX) * (ny / TC_TY);
+// Levels per block: a block takes zc + 2 planes (and about one more for its weights and its last
+// epilogue), an SM holds two blocks and takes their planes one after another; a lone block leaves
+// gaps, about 1.6 times the time, and with 55 KB of weights a block (wbytes) more where blocks on most
+// SMs fetch them at once.  (32 -> 32 channels, us: 128x128x64 with 5 levels 125, 10: 103, 32, which this
+// picks: 96; 64^3 4: 43, 8, picked: 36, 16: 43; 64x64x32 4, picked: 25, 8: 27; a corrected step at
+// 32^3 with 2 levels 154.4, 3, picked: 151.9, 4: 155.3.)
+int tc_levels(int tiles, int nz, int sms, int wbytes) {
   int zc = nz;
   double best = -1.0;
-  for (int nch = 1; nch <= (nz + 3) / 4; ++nch) {
+  for (int nch = 1; nch <= nz; ++nch) {
     const int z = (nz + nch - 1) / nch;
-    const long long blocks = (long long)tiles * ((nz + z - 1) / z);
-    const double fill = (double)blocks / ((double)((blocks + cap - 1) / cap) * cap);
-    if (fill > best + 1e-9) {
-      best = fill;
+    const long long blocks = (long long)tiles * ((nz + z - 1) / z), per_sm = (blocks + sms - 1) / sms;
+    const double alone = wbytes > 32 * 1024 && 3 * blocks > 2 * sms ? 2.0 : 1.6;
+    const double cost = (z + 3) * (per_sm == 1 ? alone : (double)per_sm);
+    if (best < 0 || cost < best) {
+      best = cost;
       zc = z;
     }
   }
+  return zc;
+}
+
+template <int CIN, int COUT>
+cudaError_t launch_tc(int nx, int ny, int nz, const void* x, const __nv_bfloat16* w, const ConvEpilogue& o,
+                      cudaStream_t st, bool pdl) {
+  int sms = 0;
+  cudaError_t e = tc_setup<CIN, COUT>(&sms);
+  if (e != cudaSuccess) return e;
+  CUtensorMap xmap;
+  if (!make_xmap(&xmap, x, nx, ny, nz, CIN)) return cudaErrorInvalidValue;
+  using L = TcLayout<CIN, COUT>;
+  const int tiles = (nx / TC_TX) * (ny / TC_TY), zc = tc_levels(tiles, nz, sms, L::W_BYTES);
   if ((long long)tiles * ((nz + zc - 1) / zc) > 0x7fffffffll) return cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(tiles * ((nz + zc - 1) / zc)));
@@ -736,8 +866,7 @@ cudaError_t launch_tc(int nx, int ny, int nz, const void* x, const __nv_bfloat16
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, k_conv3d_tc<CIN, COUT>, xmap, nx, ny, nz, zc, w, bias, pre, ybf, yf, gelu, creal,
-                            pdl ? 1 : 0);
+  return cudaLaunchKernelEx(&cfg, k_conv3d_tc<CIN, COUT>, xmap, nx, ny, nz, zc, w, o, pdl ? 1 : 0);
 }
 
 
@@ -828,19 +957,18 @@ cudaError_t launch_dw(int nx, int ny, int nz, int cin, int cout, const void* x, 
 }
 }  // namespace
 
-bool conv_tc_fits(int nx, int ny, int nz, int cin, int cout, const void* x, const void* pre, const void* ybf,
-                  const void* yf) {
-  const uintptr_t align = (uintptr_t)x | (uintptr_t)pre | (uintptr_t)ybf | (uintptr_t)yf;   // 16-byte TMA / stores
+bool conv_tc_fits(int nx, int ny, int nz, int cin, int cout, const void* x, const ConvEpilogue& o) {
+  const uintptr_t align = (uintptr_t)x | (uintptr_t)o.pre | (uintptr_t)o.ybf | (o.compact ? 0 : (uintptr_t)o.yf) |
+                          (uintptr_t)o.gpre;   // 16-byte TMA / loads / stores
   return (cin == 16 || cin == 32) && (cout == 8 || cout == 16 || cout == 32) && nx > 0 && ny > 0 && nz > 0 &&
          nx % TC_TX == 0 && ny % TC_TY == 0 && (align & 15) == 0 && tc_encoder() != nullptr;
 }
 
-cudaError_t launch_conv_tc(int nx, int ny, int nz, int cin, int cout, const void* x, const void* w, const float* bias,
-                           float* pre, void* ybf, float* yf, int gelu, int creal, cudaStream_t st, bool pdl) {
-  if (!conv_tc_fits(nx, ny, nz, cin, cout, x, pre, ybf, yf)) return cudaErrorInvalidValue;
+cudaError_t launch_conv_tc(int nx, int ny, int nz, int cin, int cout, const void* x, const void* w,
+                           const ConvEpilogue& o, cudaStream_t st, bool pdl) {
+  if (!conv_tc_fits(nx, ny, nz, cin, cout, x, o)) return cudaErrorInvalidValue;
   const __nv_bfloat16* wb = (const __nv_bfloat16*)w;
-  __nv_bfloat16* yb = (__nv_bfloat16*)ybf;
-#define LEXGB_TC(CI, CO) launch_tc<CI, CO>(nx, ny, nz, x, wb, bias, pre, yb, yf, gelu, creal, st, pdl)
+#define LEXGB_TC(CI, CO) launch_tc<CI, CO>(nx, ny, nz, x, wb, o, st, pdl)
   if (cin == 16) return cout == 8 ? LEXGB_TC(16, 8) : cout == 16 ? LEXGB_TC(16, 16) : LEXGB_TC(16, 32);
   return cout == 8 ? LEXGB_TC(32, 8) : cout == 16 ? LEXGB_TC(32, 16) : LEXGB_TC(32, 32);
 #undef LEXGB_TC
@@ -849,12 +977,12 @@ cudaError_t launch_conv_tc(int nx, int ny, int nz, int cin, int cout, const void
 cudaError_t conv_tc_prepare() {
   int cap;
   cudaError_t e;
-  if ((e = tc_grid<16, 8>(&cap)) != cudaSuccess) return e;
-  if ((e = tc_grid<16, 16>(&cap)) != cudaSuccess) return e;
-  if ((e = tc_grid<16, 32>(&cap)) != cudaSuccess) return e;
-  if ((e = tc_grid<32, 8>(&cap)) != cudaSuccess) return e;
-  if ((e = tc_grid<32, 16>(&cap)) != cudaSuccess) return e;
-  if ((e = tc_grid<32, 32>(&cap)) != cudaSuccess) return e;
+  if ((e = tc_setup<16, 8>(&cap)) != cudaSuccess) return e;
+  if ((e = tc_setup<16, 16>(&cap)) != cudaSuccess) return e;
+  if ((e = tc_setup<16, 32>(&cap)) != cudaSuccess) return e;
+  if ((e = tc_setup<32, 8>(&cap)) != cudaSuccess) return e;
+  if ((e = tc_setup<32, 16>(&cap)) != cudaSuccess) return e;
+  if ((e = tc_setup<32, 32>(&cap)) != cudaSuccess) return e;
   if ((e = dw_grid<2, 16>(&cap)) != cudaSuccess) return e;
   if ((e = dw_grid<2, 32>(&cap)) != cudaSuccess) return e;
   if ((e = dw_grid<4, 16>(&cap)) != cudaSuccess) return e;

@@ -370,9 +370,10 @@ cudaError_t launch_smag_b(const Dims&, const Phys&, const Cols&, State in, SmagT
 
 // learned SGS correction: network input from the state (16 BF16 channels a cell) and the
 // correction (8 FP32 channels a cell, 5 used) scaled and added back to the state
-cudaError_t launch_sgs_pack(int nx, int ny, int nz, const float* T, const float* u, const float* v, const float* w,
-                            const float* q, float theta_ref, const float* lo, const float* rin, void* x16,
-                            cudaStream_t);
+// the input and the first layer together: w0, b0 its weights and biases, out its output (32 channels)
+cudaError_t launch_sgs_input(int nx, int ny, int nz, const float* T, const float* u, const float* v, const float* w,
+                             const float* q, float theta_ref, const float* lo, const float* rin, void* x16,
+                             const void* w0, const float* b0, void* out, cudaStream_t, bool pdl);
 cudaError_t conv_prepare();  // one-time set-up of the CNN convolution kernels (outside graph capture)
 // one convolution (cin 16 or 32, cout 8, 16 or 32); pdl: launched as a programmatic dependent of
 // the previous kernel of the stream, which must not write w or bias

@@ -5,9 +5,10 @@ library's BF16 tensor-core kernels, as a torch.autograd operation.
       -> conv 32->32, GELU -> conv 32->5 -> correction (5 fields)
 
 All convolutions are 3x3x3 with zero padding ('SAME'), biases on, tanh-GELU (flax ``nn.gelu``).
-The forward runs ``lexgb_cnn_conv3d`` (BF16 operands, FP32 accumulation); the backward runs the
-same kernel on the mirrored, transposed weights for the input gradients, ``lexgb_cnn_gelu_bwd``
-and ``lexgb_cnn_conv3d_dw`` for the weight and bias gradients.  ``adam_step`` updates the FP32
+The forward is one library call (``lexgb_cnn_net_forward``: BF16 operands, FP32 accumulation), the
+backward another (``lexgb_cnn_net_backward``): the same convolutions on the mirrored, transposed
+weights for the input gradients, with GELU' and the bias sums in their epilogue, and the
+weight-gradient kernel.  ``adam_step`` updates the FP32
 master weights with ``lexgb_cnn_adam`` (the reference uses optax.lamb, lex_dl_train.py).
 
 Packing, as the reference's (dl_models.py:125-182, one_sprint_functions.py:136-151): theta, u, v, w,
@@ -92,9 +93,8 @@ def conv3d(x_bf16, w_bf16, bias, nx, ny, nz, cin, cout, gelu, creal, want_pre=Tr
     return pre, ybf, yf
 
 
-def _mirror(w_bf16):
-    """[27][cout][cin] -> [27][cin][cout] with the offsets reversed: the input-gradient weights."""
-    return w_bf16.flip(0).transpose(1, 2).contiguous()
+def _ptrs(tensors):
+    return (ctypes.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
 
 
 def _pad_channels(t, c):
@@ -105,58 +105,46 @@ def _pad_channels(t, c):
     return out
 
 
+WSIZES = [27 * cout * cin for cin, cout, _ in LAYERS]
+GRAD_WORK = sum(27 * cin * (16 if cout == 8 else 32) for cin, cout, _ in LAYERS)   # mirrored weights
+
+
 class _NetFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, net, dims, *params):
         nx, ny, nz = dims
-        a = _pad_channels(x.to(torch.bfloat16), 16)
-        acts, pres = [a], []
-        for li, (cin, cout, gelu) in enumerate(LAYERS):
-            last = li == len(LAYERS) - 1
-            pre, ybf, yf = conv3d(acts[-1], net.wbf[li], net.b[li], nx, ny, nz, cin, cout, gelu,
-                                  COUT_REAL if last else cout, want_pre=not last, out_f32=last)
-            pres.append(pre)
-            if not last:
-                acts.append(ybf)
-            else:
-                out = yf[:, :COUT_REAL].contiguous()
+        n = nx * ny * nz
+        if x.shape[0] < n:
+            raise ValueError("x must have at least nx*ny*nz = %d rows, got %d" % (n, x.shape[0]))
+        five = x.shape[1] == CIN0
+        if five:      # rounded to BF16 by the first kernel
+            a0 = torch.empty(n, 16, device="cuda", dtype=torch.bfloat16)
+            xin = x if x.dtype == torch.float32 else x.to(torch.bfloat16).float()
+            xin = xin.contiguous()
+        else:
+            a0, xin = _pad_channels(x.to(torch.bfloat16), 16), None
+        acts = [a0] + list(torch.empty(3, n, C, device="cuda", dtype=torch.bfloat16))
+        pres = list(torch.empty(3, n, C, device="cuda"))
+        out = torch.empty(n, COUT_REAL, device="cuda")
+        _lib.check(_lib.load().lexgb_cnn_net_forward(nx, ny, nz, _p(xin), _ptrs(net.wbf), _ptrs(net.b), _ptrs(acts),
+                                                     _ptrs(pres), _p(out), _stream()))
         ctx.net, ctx.dims, ctx.acts, ctx.pres = net, dims, acts, pres
         return out
 
     @staticmethod
     def backward(ctx, gout):
         net, (nx, ny, nz) = ctx.net, ctx.dims
-        lib = _lib.load()
         n = nx * ny * nz
-        st = _stream()
-        # gradient at the last layer's output: no GELU; channels padded to 16 for the input-gradient conv
-        dy = _pad_channels(gout.float().contiguous(), 8)
-        g = torch.empty(n, 16, device="cuda", dtype=torch.bfloat16)
-        _lib.check(lib.lexgb_cnn_gelu_bwd(n, 8, 16, _p(dy), None, _p(g), st))
-        gstride = 16
-        grads_w = [None] * len(LAYERS)
-        grads_b = [None] * len(LAYERS)
-        dx = None
-        for li in range(len(LAYERS) - 1, -1, -1):
-            cin, cout, _ = LAYERS[li]
-            dw = torch.zeros(27, cout, cin, device="cuda")
-            db = torch.zeros(cout, device="cuda")
-            _lib.check(lib.lexgb_cnn_conv3d_dw(nx, ny, nz, cin, cout, gstride, _p(ctx.acts[li]), _p(g), _p(dw),
-                                               _p(db), st))
-            grads_w[li], grads_b[li] = dw, db
-            # input gradient: mirrored weights, padded so that the gradient's channels are the k16 input
-            wm = _mirror(net.wbf[li])                       # [27][cin][cout]
-            if gstride != cout:
-                wm = torch.cat([wm, torch.zeros(27, cin, gstride - cout, device="cuda", dtype=wm.dtype)], 2)
-            _, _, da = conv3d(g, wm.contiguous(), None, nx, ny, nz, gstride, cin, False, cin,
-                              want_pre=False, out_f32=True)
-            if li == 0:
-                dx = da[:, :CIN0].contiguous()
-                break
-            g = torch.empty(n, cin, device="cuda", dtype=torch.bfloat16)
-            _lib.check(lib.lexgb_cnn_gelu_bwd(n, cin, cin, _p(da), _p(ctx.pres[li - 1]), _p(g), st))
-            gstride = cin
-        return (dx, None, None) + tuple(grads_w) + tuple(grads_b)
+        gout = gout.float().contiguous()
+        work = torch.empty(64 * n + GRAD_WORK, device="cuda", dtype=torch.bfloat16)
+        nb = [cout for _, cout, _ in LAYERS]
+        grads = torch.empty(sum(WSIZES) + sum(nb), device="cuda")
+        dx = torch.empty(n, CIN0, device="cuda")
+        _lib.check(_lib.load().lexgb_cnn_net_backward(nx, ny, nz, _p(gout), _ptrs(net.wbf), _ptrs(ctx.acts),
+                                                      _ptrs(ctx.pres), _p(work), _p(grads), _p(dx), _stream()))
+        parts = torch.split(grads, WSIZES + nb)
+        dw = tuple(g.view(27, cout, cin) for g, (cin, cout, _) in zip(parts, LAYERS))
+        return (dx, None, None) + dw + tuple(parts[4:])
 
 
 def net_apply(net, x, dims):

@@ -120,6 +120,9 @@ struct lexgb_ctx {
   // graph of one big step
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
+  // graphs of the reverse mode's passes (run_adjoint), and the passes run since the last drop_graph
+  cudaGraphExec_t adj_exec[3]{};
+  int adj_runs[3]{};
 };
 
 namespace {
@@ -354,6 +357,11 @@ void drop_graph(lexgb_ctx* c) {
   if (c->graph) cudaGraphDestroy(c->graph);
   c->gexec = nullptr;
   c->graph = nullptr;
+  for (int i = 0; i < 3; ++i) {
+    if (c->adj_exec[i]) cudaGraphExecDestroy(c->adj_exec[i]);
+    c->adj_exec[i] = nullptr;
+    c->adj_runs[i] = 0;
+  }
 }
 
 int build_table(lexgb_ctx* c) {
@@ -1231,8 +1239,58 @@ bool l2_window_for(lexgb_ctx* c, void* base, size_t bytes, cudaAccessPolicyWindo
   return true;
 }
 
-int zero_state(lexgb_ctx* c, const State& s) {
-  for (int f = 0; f < NFIELD; ++f) CK(cudaMemsetAsync(field_of(s, f), 0, c->fstride * sizeof(float), c->stream));
+// n adjacent fields of the workspace
+int zero_fields(lexgb_ctx* c, float* base, int n) {
+  CK(cudaMemsetAsync(base, 0, (size_t)n * c->fstride * sizeof(float), c->stream));
+  return LEXGB_OK;
+}
+
+// the persisting windows of the reverse mode's acoustic loops
+struct AdjWindows {
+  bool fwd_on[3], rev_on;
+  cudaAccessPolicyWindow fwd[3], rev;
+};
+AdjWindows adj_windows(lexgb_ctx* c, AdjWork& w, int nstages) {
+  AdjWindows a{};
+  // the stage's theta_rho, R_u, R_v, R_w (adjacent workspace fields) persist in L2 through its sub-steps
+  for (int s = 0; s < nstages; ++s) a.fwd_on[s] = l2_window_for(c, w.trho[s], 4 * c->fstride * sizeof(float), &a.fwd[s]);
+  // the acoustic adjoints read and write the five accumulators (adjacent fields) in every sub-step
+  a.rev_on = l2_window_for(c, w.Rub, 5 * c->fstride * sizeof(float), &a.rev);
+  return a;
+}
+
+// A pass of the reverse mode (about 150 launches): on the third run with the same settings and from then on
+// as one graph, launched on the bound stream.  A launch a kernel held small grids up: 64x64x64, two steps
+// and their reverse pass, 4.2 ms of which the GPU worked 2.9, as graphs 3.3 ms.  Not on the first runs, as
+// a constant that is learned changes the settings on every step, and the capture costs about as much as the
+// launches; not while the caller captures the bound stream.
+enum { ADJ_KEEP, ADJ_KEPT, ADJ_RECOMPUTED };
+extern "C++" template <class F>
+int run_adjoint(lexgb_ctx* c, int which, const F& pass) {
+  if (!c->adj_exec[which]) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess) {
+      cudaGetLastError();
+      return pass();
+    }
+    if (cap != cudaStreamCaptureStatusNone || ++c->adj_runs[which] < 3) return pass();
+    cudaStream_t bound = c->stream;
+    c->stream = c->own_stream;   // as the step graph: the legacy default stream cannot be captured
+    cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) {
+      c->stream = bound;
+      return fail(LEXGB_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+    }
+    const int st = pass();
+    cudaGraph_t g = nullptr;
+    e = cudaStreamEndCapture(c->stream, &g);
+    c->stream = bound;
+    if (st == LEXGB_OK && e == cudaSuccess) e = cudaGraphInstantiate(&c->adj_exec[which], g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (st != LEXGB_OK) return st;
+    if (e != cudaSuccess) return fail(LEXGB_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+  }
+  CK(cudaGraphLaunch(c->adj_exec[which], c->stream));
   return LEXGB_OK;
 }
 
@@ -1241,7 +1299,7 @@ int zero_state(lexgb_ctx* c, const State& s) {
 namespace {
 
 // forward of the first nstages stages from x0, keeping every intermediate the reverse pass reads
-int adj_forward(lexgb_ctx* c, AdjWork& w, const State& x0, int nstages) {
+int adj_forward(lexgb_ctx* c, AdjWork& w, const AdjWindows& win, const State& x0, int nstages) {
   const Dims& d = c->d;
   const StagePlan p = plan_of(c->cfg);
   const State& A = x0;
@@ -1258,45 +1316,36 @@ int adj_forward(lexgb_ctx* c, AdjWork& w, const State& x0, int nstages) {
                           w.trho[s]));
     CK(launch_adv_momentum(d, c->ph, c->cols, xs, w.div[s], sg, w.Ru[s], w.Rv[s], w.Rw[s], 0, c->stream));
     AcousticIn in{A.u, A.v, A.w, A.p, w.Ru[s], w.Rv[s], w.Rw[s], w.trho[s], xs.p};
-    // the stage's theta_rho, R_u, R_v, R_w (adjacent workspace fields) persist in L2 through its sub-steps
-    cudaAccessPolicyWindow win{};
-    const bool win_on = l2_window_for(c, w.trho[s], 4 * c->fstride * sizeof(float), &win);
     for (int m = 1; m <= p.n[s]; ++m) {
       const AcousticOut o{w.ac[s][m][0], w.ac[s][m][1], w.ac[s][m][2], w.ac[s][m][3]};
-      CK(sub_step(c, in, o, (float)p.dtau[s], 0, win_on ? &win : nullptr));
+      CK(sub_step(c, in, o, (float)p.dtau[s], 0, win.fwd_on[s] ? &win.fwd[s] : nullptr));
       in.u = o.u; in.v = o.v; in.w = o.w; in.p = o.p;
     }
   }
   return LEXGB_OK;
 }
 
-// reverse pass over the intermediates adj_forward kept for x0
-int adj_reverse(lexgb_ctx* c, AdjWork& w, const State& x0, int nstages, const float* const ybar[6], float* xbar[6],
-                int on_device) {
+// The reverse pass's seed, in w.Cur.  (Outside the captured pass: the caller's pointers.)
+int adj_seed(lexgb_ctx* c, AdjWork& w, const float* const ybar[6], int on_device) {
+  CKS(zero_fields(c, w.Cur.T, NFIELD));
+  for (int f = 0; f < 6; ++f)
+    CK(cudaMemcpyAsync(field_of(w.Cur, f), ybar[f], (size_t)(f == 3 ? c->d.faces() : c->d.cells()) * sizeof(float),
+                       on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c->stream));
+  return LEXGB_OK;
+}
+
+// reverse pass over the intermediates adj_forward kept for x0, from w.Cur to w.Xb0
+int adj_reverse(lexgb_ctx* c, AdjWork& w, const AdjWindows& win, const State& x0, int nstages) {
   const Dims& d = c->d;
   const StagePlan p = plan_of(c->cfg);
   const State& A = x0;
   const bool turb = c->cfg.turb_opt == 1;
-  // ---- seed
-  const size_t cells = (size_t)d.cells(), faces = (size_t)d.faces();
-  for (int f = 0; f < 6; ++f) {
-    const size_t n = (f == 3 ? faces : cells) * sizeof(float);
-    CK(cudaMemsetAsync(field_of(w.Cur, f), 0, c->fstride * sizeof(float), c->stream));
-    CK(cudaMemcpyAsync(field_of(w.Cur, f), ybar[f], n, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
-                       c->stream));
-  }
-  CKS(zero_state(c, w.Xb0));
-  if (turb)
-    for (int f = 0; f < 5; ++f) CK(cudaMemsetAsync(w.sgsb[f], 0, c->fstride * sizeof(float), c->stream));
-  // ---- reverse.  The acoustic adjoints read and write the five accumulators (adjacent fields)
-  // in every sub-step: a persisting L2 window keeps them on chip through a stage.
-  cudaAccessPolicyWindow awin{};
-  const bool awin_on = l2_window_for(c, w.Rub, 5 * c->fstride * sizeof(float), &awin);
+  CKS(zero_fields(c, w.Xb0.T, NFIELD));
+  if (turb) CKS(zero_fields(c, w.sgsb[0], 5));
   for (int s = nstages - 1; s >= 0; --s) {
     const State xs = s == 0 ? A : w.S[s];
-    CKS(zero_state(c, w.Xs));
-    for (float* z : {w.Rub, w.Rvb, w.Rwb, w.trhob, w.psb})
-      CK(cudaMemsetAsync(z, 0, c->fstride * sizeof(float), c->stream));
+    CKS(zero_fields(c, w.Xs.T, NFIELD));
+    CKS(zero_fields(c, w.Rub, 5));
     // acoustic loop backwards
     const float* adj[4] = {w.Cur.u, w.Cur.v, w.Cur.w, w.Cur.p};
     for (int m = p.n[s], k = 0; m >= 1; --m, ++k) {
@@ -1305,7 +1354,7 @@ int adj_reverse(lexgb_ctx* c, AdjWork& w, const State& x0, int nstages, const fl
       AcousticVjpArgs a{oldp, w.trho[s], xs.p, w.ac[s][m][0], w.ac[s][m][1], w.ac[s][m][2],
                         adj[0], adj[1], adj[2], adj[3], o[0], o[1], o[2], o[3],
                         w.Rub, w.Rvb, w.Rwb, w.trhob, w.psb};
-      CK(launch_acoustic_vjp(d, c->ph, c->cols, a, (float)p.dtau[s], c->stream, awin_on ? &awin : nullptr));
+      CK(launch_acoustic_vjp(d, c->ph, c->cols, a, (float)p.dtau[s], c->stream, win.rev_on ? &win.rev : nullptr));
       for (int f = 0; f < 4; ++f) adj[f] = o[f];
     }
     // slow tendencies, theta/qv update, theta_rho, pi'_s; the acoustic loop's input adjoints go to
@@ -1347,15 +1396,17 @@ int adj_reverse(lexgb_ctx* c, AdjWork& w, const State& x0, int nstages, const fl
     // dK_m/dCs = 2 K_m / Cs: the Cs derivative of this step
     CK(launch_sum_scaled(d.cells(), w.sv.kmkb, 2.0 / c->cs, c->cs_bar, c->stream));
   }
-  for (int f = 0; f < 6; ++f) {
-    const size_t n = (f == 3 ? faces : cells) * sizeof(float);
-    CK(cudaMemcpyAsync(xbar[f], field_of(w.Xb0, f), n, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
-                       c->stream));
-  }
+  return LEXGB_OK;
+}
+
+int adj_result(lexgb_ctx* c, AdjWork& w, const AdjWindows& win, float* xbar[6], int on_device) {
+  for (int f = 0; f < 6; ++f)
+    CK(cudaMemcpyAsync(xbar[f], field_of(w.Xb0, f), (size_t)(f == 3 ? c->d.faces() : c->d.cells()) * sizeof(float),
+                       on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   // the accumulators' persisting lines (71 MB at 192 x 192 x 96) would crowd the L2 of the work
   // that follows; return them to normal use (the step's own window re-persists its fields)
-  if (awin_on) cudaCtxResetPersistingL2Cache();
+  if (win.rev_on) cudaCtxResetPersistingL2Cache();
   return LEXGB_OK;
 }
 
@@ -1376,8 +1427,17 @@ int lexgb_step_vjp(lexgb_ctx* c, int nstages, const float* const ybar[6], float*
   AdjWork w;
   CKS(ensure_adjoint(c, w));
   c->adj_kept = false;  // the workspace is reused below
-  CKS(adj_forward(c, w, c->A, nstages));
-  return adj_reverse(c, w, c->A, nstages, ybar, xbar, on_device);
+  const AdjWindows win = adj_windows(c, w, nstages);
+  CKS(adj_seed(c, w, ybar, on_device));
+  auto pass = [&] {
+    CKS(adj_forward(c, w, win, c->A, nstages));
+    return adj_reverse(c, w, win, c->A, nstages);
+  };
+  if (nstages == 3)
+    CKS(run_adjoint(c, ADJ_RECOMPUTED, pass));
+  else
+    CKS(pass());
+  return adj_result(c, w, win, xbar, on_device);
 }
 
 int lexgb_step_keep(lexgb_ctx* c) {
@@ -1388,7 +1448,8 @@ int lexgb_step_keep(lexgb_ctx* c) {
   for (int f = 0; f < NFIELD; ++f)
     CK(cudaMemcpyAsync(field_of(w.X0, f), field_of(c->A, f), c->fstride * sizeof(float), cudaMemcpyDeviceToDevice,
                        c->stream));
-  CKS(adj_forward(c, w, w.X0, 3));
+  const AdjWindows win = adj_windows(c, w, 3);
+  CKS(run_adjoint(c, ADJ_KEEP, [&] { return adj_forward(c, w, win, w.X0, 3); }));
   for (int f = 0; f < NFIELD; ++f)
     CK(cudaMemcpyAsync(field_of(c->A, f), field_of(w.S[3], f), c->fstride * sizeof(float), cudaMemcpyDeviceToDevice,
                        c->stream));
@@ -1403,7 +1464,10 @@ int lexgb_step_vjp_kept(lexgb_ctx* c, const float* const ybar[6], float* xbar[6]
   if (!c->adj_kept) return fail(LEXGB_ERR_STATE, "no kept step: call lexgb_step_keep first");
   AdjWork w;
   CKS(ensure_adjoint(c, w));
-  return adj_reverse(c, w, w.X0, 3, ybar, xbar, on_device);
+  const AdjWindows win = adj_windows(c, w, 3);
+  CKS(adj_seed(c, w, ybar, on_device));
+  CKS(run_adjoint(c, ADJ_KEPT, [&] { return adj_reverse(c, w, win, w.X0, 3); }));
+  return adj_result(c, w, win, xbar, on_device);
 }
 
 int lexgb_last_error(char* buf, size_t len) {

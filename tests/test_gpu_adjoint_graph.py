@@ -1,0 +1,54 @@
+"""The reverse mode's passes as graphs (from their third run on) against the same passes launched one kernel
+at a time: repeated runs agree bit for bit, on another stream too, and a changed constant is taken up."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _solver(nx, ny, nz):
+    from lex_gb300.solver import Solver
+    from lex_gb300.workload import warm_bubble
+    phys, prof = warm_bubble(nx, ny, nz, 300.0, 300.0, 300.0, amplitude=2.0, radius_h=1500.0, seed=3)
+    S = Solver(nx, ny, nz, 300.0, 300.0, 300.0, 1.5, 32, turb_opt=1)
+    S.integrate_base_state(prof["theta0"], prof["qv0"])
+    S.upload(phys, dtype=np.float32)
+    S.step(3)
+    return S
+
+
+@pytest.mark.parametrize("dims", [(16, 12, 9), (30, 11, 8)], ids=str)
+def test_repeated_reverse_passes_agree(built_lib, dims):
+    torch = pytest.importorskip("torch")
+    from lex_gb300 import autograd as lag
+    with _solver(*dims) as S:
+        x0 = lag.get_state(S)
+        g = torch.Generator(device="cpu").manual_seed(1)
+        seeds = [torch.randn(t.shape, generator=g).cuda() for t in x0]
+
+        def run(cs):
+            x = [t.detach().clone().requires_grad_(True) for t in x0]
+            c = torch.tensor(cs, device="cuda", requires_grad=True)
+            y = lag.rollout(S, x, 2, cs=c)          # the second step is kept, the first recomputed
+            return list(y) + list(torch.autograd.grad(y, x + [c], grad_outputs=seeds))
+
+        def same(a, b):
+            for i, (p, q) in enumerate(zip(a[:-1], b[:-1])):
+                assert torch.equal(p, q), i
+            # the constant's gradient is summed in FP64 by atomic additions of the blocks' sums
+            assert abs(float(a[-1] - b[-1])) <= 1e-9 * abs(float(a[-1])) + 1e-12
+        first = run(0.18)
+        for _ in range(4):
+            same(first, run(0.18))
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            again = run(0.18)
+        torch.cuda.current_stream().wait_stream(side)
+        side.synchronize()
+        same(first, again)
+        other = run(0.25)
+        assert not torch.equal(other[0], first[0]) or not torch.equal(other[6], first[6])
+        for _ in range(4):
+            same(other, run(0.25))
+        same(first, run(0.18))

@@ -1245,17 +1245,17 @@ int zero_fields(lexgb_ctx* c, float* base, int n) {
   return LEXGB_OK;
 }
 
-// the persisting windows of the reverse mode's acoustic loops
+// the persisting windows of the forward pass's acoustic loops: a stage's theta_rho, R_u, R_v, R_w (adjacent
+// workspace fields) persist in L2 through its sub-steps (a rollout and its reverse pass: 192x192x96 10.62 ->
+// 10.33 ms, 128x128x64 3.55 -> 3.59).  The reverse pass's five accumulators do not: their window took more
+// than half of the L2 from the other ten fields of a sub-step (192x192x96 10.83 ms with it, 10.64 without).
 struct AdjWindows {
-  bool fwd_on[3], rev_on;
-  cudaAccessPolicyWindow fwd[3], rev;
+  bool on[3];
+  cudaAccessPolicyWindow win[3];
 };
 AdjWindows adj_windows(lexgb_ctx* c, AdjWork& w, int nstages) {
   AdjWindows a{};
-  // the stage's theta_rho, R_u, R_v, R_w (adjacent workspace fields) persist in L2 through its sub-steps
-  for (int s = 0; s < nstages; ++s) a.fwd_on[s] = l2_window_for(c, w.trho[s], 4 * c->fstride * sizeof(float), &a.fwd[s]);
-  // the acoustic adjoints read and write the five accumulators (adjacent fields) in every sub-step
-  a.rev_on = l2_window_for(c, w.Rub, 5 * c->fstride * sizeof(float), &a.rev);
+  for (int s = 0; s < nstages; ++s) a.on[s] = l2_window_for(c, w.trho[s], 4 * c->fstride * sizeof(float), &a.win[s]);
   return a;
 }
 
@@ -1318,7 +1318,7 @@ int adj_forward(lexgb_ctx* c, AdjWork& w, const AdjWindows& win, const State& x0
     AcousticIn in{A.u, A.v, A.w, A.p, w.Ru[s], w.Rv[s], w.Rw[s], w.trho[s], xs.p};
     for (int m = 1; m <= p.n[s]; ++m) {
       const AcousticOut o{w.ac[s][m][0], w.ac[s][m][1], w.ac[s][m][2], w.ac[s][m][3]};
-      CK(sub_step(c, in, o, (float)p.dtau[s], 0, win.fwd_on[s] ? &win.fwd[s] : nullptr));
+      CK(sub_step(c, in, o, (float)p.dtau[s], 0, win.on[s] ? &win.win[s] : nullptr));
       in.u = o.u; in.v = o.v; in.w = o.w; in.p = o.p;
     }
   }
@@ -1335,7 +1335,7 @@ int adj_seed(lexgb_ctx* c, AdjWork& w, const float* const ybar[6], int on_device
 }
 
 // reverse pass over the intermediates adj_forward kept for x0, from w.Cur to w.Xb0
-int adj_reverse(lexgb_ctx* c, AdjWork& w, const AdjWindows& win, const State& x0, int nstages) {
+int adj_reverse(lexgb_ctx* c, AdjWork& w, const State& x0, int nstages) {
   const Dims& d = c->d;
   const StagePlan p = plan_of(c->cfg);
   const State& A = x0;
@@ -1353,8 +1353,8 @@ int adj_reverse(lexgb_ctx* c, AdjWork& w, const AdjWindows& win, const State& x0
       const float* oldp = m == 1 ? A.p : w.ac[s][m - 1][3];
       AcousticVjpArgs a{oldp, w.trho[s], xs.p, w.ac[s][m][0], w.ac[s][m][1], w.ac[s][m][2],
                         adj[0], adj[1], adj[2], adj[3], o[0], o[1], o[2], o[3],
-                        w.Rub, w.Rvb, w.Rwb, w.trhob, w.psb};
-      CK(launch_acoustic_vjp(d, c->ph, c->cols, a, (float)p.dtau[s], c->stream, win.rev_on ? &win.rev : nullptr));
+                        w.Rub, w.Rvb, w.Rwb, w.trhob, w.psb, k & 1 ? 2 : m == 1 ? 1 : 0};
+      CK(launch_acoustic_vjp(d, c->ph, c->cols, a, (float)p.dtau[s], c->stream));
       for (int f = 0; f < 4; ++f) adj[f] = o[f];
     }
     // slow tendencies, theta/qv update, theta_rho, pi'_s; the acoustic loop's input adjoints go to
@@ -1399,14 +1399,11 @@ int adj_reverse(lexgb_ctx* c, AdjWork& w, const AdjWindows& win, const State& x0
   return LEXGB_OK;
 }
 
-int adj_result(lexgb_ctx* c, AdjWork& w, const AdjWindows& win, float* xbar[6], int on_device) {
+int adj_result(lexgb_ctx* c, AdjWork& w, float* xbar[6], int on_device) {
   for (int f = 0; f < 6; ++f)
     CK(cudaMemcpyAsync(xbar[f], field_of(w.Xb0, f), (size_t)(f == 3 ? c->d.faces() : c->d.cells()) * sizeof(float),
                        on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  // the accumulators' persisting lines (71 MB at 192 x 192 x 96) would crowd the L2 of the work
-  // that follows; return them to normal use (the step's own window re-persists its fields)
-  if (win.rev_on) cudaCtxResetPersistingL2Cache();
   return LEXGB_OK;
 }
 
@@ -1431,13 +1428,13 @@ int lexgb_step_vjp(lexgb_ctx* c, int nstages, const float* const ybar[6], float*
   CKS(adj_seed(c, w, ybar, on_device));
   auto pass = [&] {
     CKS(adj_forward(c, w, win, c->A, nstages));
-    return adj_reverse(c, w, win, c->A, nstages);
+    return adj_reverse(c, w, c->A, nstages);
   };
   if (nstages == 3)
     CKS(run_adjoint(c, ADJ_RECOMPUTED, pass));
   else
     CKS(pass());
-  return adj_result(c, w, win, xbar, on_device);
+  return adj_result(c, w, xbar, on_device);
 }
 
 int lexgb_step_keep(lexgb_ctx* c) {
@@ -1464,10 +1461,9 @@ int lexgb_step_vjp_kept(lexgb_ctx* c, const float* const ybar[6], float* xbar[6]
   if (!c->adj_kept) return fail(LEXGB_ERR_STATE, "no kept step: call lexgb_step_keep first");
   AdjWork w;
   CKS(ensure_adjoint(c, w));
-  const AdjWindows win = adj_windows(c, w, 3);
   CKS(adj_seed(c, w, ybar, on_device));
-  CKS(run_adjoint(c, ADJ_KEPT, [&] { return adj_reverse(c, w, win, w.X0, 3); }));
-  return adj_result(c, w, win, xbar, on_device);
+  CKS(run_adjoint(c, ADJ_KEPT, [&] { return adj_reverse(c, w, w.X0, 3); }));
+  return adj_result(c, w, xbar, on_device);
 }
 
 int lexgb_last_error(char* buf, size_t len) {

@@ -251,56 +251,13 @@ __device__ __forceinline__ AcCol acoustic_col(const Cols& c, int k, int nz) {
   return q;
 }
 
-// one thread per cell (any nx)
-__global__ void __launch_bounds__(AB) k_acoustic_vjp(Dims d, Phys ph, Cols c, AcousticVjpArgs a, float dtau) {
-  const long long t = (long long)blockIdx.x * AB + threadIdx.x;
-  const int nx = d.nx, ny = d.ny, nz = d.nz, plane = d.plane();
-  if (t >= d.cells()) return;
-  const int i = (int)(t % nx), j = (int)((t / nx) % ny), k = (int)(t / plane);
-  const int id = (int)t, row = k * plane + j * nx;
-  const AcCol col = acoustic_col(c, k, nz);
-  int q[7];
-  q[0] = id;
-  q[1] = row + wrapx(i - 1, nx);
-  q[2] = row + wrapx(i + 1, nx);
-  q[3] = k * plane + wrapx(j - 1, ny) * nx + i;
-  q[4] = k * plane + wrapx(j + 1, ny) * nx + i;
-  q[5] = col.hb ? id - plane : id;
-  q[6] = col.ht ? id + plane : id;
-  const float K = kDivDamp * dtau;
-  AcNbr n;
-#pragma unroll
-  for (int m = 0; m < 7; ++m) {
-    const bool ok = (m < 5) || (m == 5 ? col.hb : col.ht);
-    n.A[m] = ok ? K * LD(a.pnb, q[m]) : 0.f;
-    n.s[m] = ok ? LD(a.ps, q[m]) : 0.f;
-    n.p[m] = ok ? LD(a.p, q[m]) : 0.f;
-    n.t[m] = ok ? LD(a.trho, q[m]) : 0.f;
-  }
-  n.unb_w = LD(a.unb, id); n.unb_e = LD(a.unb, q[2]);
-  n.vnb_s = LD(a.vnb, id); n.vnb_n = LD(a.vnb, q[4]);
-  n.wnb_b = LD(a.wnb, id); n.wnb_t = LD(a.wnb, id + plane);
-  n.un_w = LD(a.un, id); n.un_e = LD(a.un, q[2]);
-  n.vn_s = LD(a.vn, id); n.vn_n = LD(a.vn, q[4]);
-  n.wn_b = LD(a.wn, id); n.wn_t = LD(a.wn, id + plane);
-  const AcOut o = acoustic_vjp_cell(n, col, LD(a.pnb, id), ph.rdx, ph.rdy, ph.rdz, dtau);
-  a.ub[id] = o.ub;
-  a.vb[id] = o.vb;
-  a.wb[id] = o.wb;
-  if (k == nz - 1) a.wb[id + plane] = 0.f;
-  a.pb[id] = o.pb;
-  a.Rub[id] += o.ub * dtau;
-  a.Rvb[id] += o.vb * dtau;
-  if (col.hb) a.Rwb[id] += o.wb * dtau;
-  a.trhob[id] += o.tb;
-  a.psb[id] += o.sb;
-}
-
-// V consecutive x cells per thread (V = 2 or 4) with V-wide row loads (nx % V == 0), as
-// k_acoustic_vec
-#ifndef ACOUSTIC_VJP_VEC
-#define ACOUSTIC_VJP_VEC 4
-#endif
+// V consecutive x cells per thread with V-wide row loads (nx % V == 0), blocks as k_acoustic_vec's.  Ten
+// fields read, four written, five accumulated: 96 bytes a cell, 84 on average with the wind accumulators
+// updated every other sub-step, from the sub-step's result and from its input, which is the result of the
+// one before.  Bound by the memory's latency (162 registers, 12 warps an SM, DRAM at 41 %): 192x192x96
+// 95 us a sub-step when the accumulators were read after the stores, and so a second trip to memory, 81 us
+// with their lines on the way to L2 from the start.  Tried: the accumulators in registers from the start
+// (198 of them: 85 us), two cells a thread and twice the warps (86), programmatic dependent launch (no gain).
 template <int V>
 struct VecF;
 template <>
@@ -311,10 +268,22 @@ template <>
 struct VecF<2> {
   typedef float2 T;
 };
+template <>
+struct VecF<1> {
+  typedef float T;
+};
 template <int V>
 __device__ __forceinline__ void ldvec(const float* p, int i, float (&o)[V]) {
   typedef typename VecF<V>::T T;
   const T t = __ldg(reinterpret_cast<const T*>(p + i));
+  const float* f = reinterpret_cast<const float*>(&t);
+#pragma unroll
+  for (int l = 0; l < V; ++l) o[l] = f[l];
+}
+template <int V>
+__device__ __forceinline__ void ldv(const float* p, int i, float (&o)[V]) {
+  typedef typename VecF<V>::T T;
+  const T t = *reinterpret_cast<const T*>(p + i);
   const float* f = reinterpret_cast<const float*>(&t);
 #pragma unroll
   for (int l = 0; l < V; ++l) o[l] = f[l];
@@ -328,23 +297,25 @@ __device__ __forceinline__ void stvec(float* p, int i, const float (&v)[V]) {
   for (int l = 0; l < V; ++l) f[l] = v[l];
   *reinterpret_cast<T*>(p + i) = t;
 }
-template <int V>
-__device__ __forceinline__ void accvec(float* p, int i, const float (&v)[V], float s) {
-  typedef typename VecF<V>::T T;
-  T t = *reinterpret_cast<T*>(p + i);
-  float* f = reinterpret_cast<float*>(&t);
-#pragma unroll
-  for (int l = 0; l < V; ++l) f[l] += v[l] * s;
-  *reinterpret_cast<T*>(p + i) = t;
-}
+__device__ __forceinline__ void prefetch_l2(const float* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+constexpr int VJP_T = 64;   // threads of a block
 
 template <int V>
-__global__ void __launch_bounds__(64) k_acoustic_vjpv(Dims d, Phys ph, Cols c, AcousticVjpArgs a, float dtau) {
+__global__ void __launch_bounds__(VJP_T) k_acoustic_vjpv(Dims d, Phys ph, Cols c, AcousticVjpArgs a, float dtau, int flat,
+                                                      int k0) {
   const int nq = d.nx / V;
-  const int qx = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z;
-  if (qx >= nq || j >= d.ny) return;
+  int qx, j;
+  if (flat) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    j = t / nq;
+    qx = t - j * nq;
+  } else {
+    qx = blockIdx.x * blockDim.x + threadIdx.x;
+    j = blockIdx.y * blockDim.y + threadIdx.y;
+  }
+  const int k = k0 + blockIdx.z;
+  if (j >= d.ny) return;
   const int nx = d.nx, ny = d.ny, nz = d.nz, plane = d.plane();
   const int i0 = V * qx;
   const int r0 = k * plane + j * nx, rs = k * plane + wrapx(j - 1, ny) * nx, rn = k * plane + wrapx(j + 1, ny) * nx;
@@ -378,6 +349,15 @@ __global__ void __launch_bounds__(64) k_acoustic_vjpv(Dims d, Phys ph, Cols c, A
   ldvec<V>(a.wn, r0 + i0, WN);
   ldvec<V>(a.wn, r0 + plane + i0, WNt);
   const float unbE = LD(a.unb, r0 + ie), unE = LD(a.un, r0 + ie);
+  // the accumulators on their way from memory while the inputs are: they are read after the results are
+  // stored, and without registers for them until then
+  if (a.acc) {
+    prefetch_l2(a.Rub + r0 + i0);
+    prefetch_l2(a.Rvb + r0 + i0);
+    prefetch_l2(a.Rwb + r0 + i0);
+  }
+  prefetch_l2(a.trhob + r0 + i0);
+  prefetch_l2(a.psb + r0 + i0);
   float ob[V], vb[V], wb[V], pb[V], tb[V], sb[V];
 #pragma unroll
   for (int l = 0; l < V; ++l) {
@@ -415,11 +395,35 @@ __global__ void __launch_bounds__(64) k_acoustic_vjpv(Dims d, Phys ph, Cols c, A
     for (int l = 0; l < V; ++l) z[l] = 0.f;
     stvec<V>(a.wb, r0 + plane + i0, z);
   }
-  accvec<V>(a.Rub, r0 + i0, ob, dtau);
-  accvec<V>(a.Rvb, r0 + i0, vb, dtau);
-  if (col.hb) accvec<V>(a.Rwb, r0 + i0, wb, dtau);
-  accvec<V>(a.trhob, r0 + i0, tb, 1.f);
-  accvec<V>(a.psb, r0 + i0, sb, 1.f);
+  float au[V], av[V], aw[V], at[V], as[V];
+  ldv<V>(a.trhob, r0 + i0, at);
+  ldv<V>(a.psb, r0 + i0, as);
+  if (a.acc) {
+    ldv<V>(a.Rub, r0 + i0, au);
+    ldv<V>(a.Rvb, r0 + i0, av);
+    ldv<V>(a.Rwb, r0 + i0, aw);
+#pragma unroll
+    for (int l = 0; l < V; ++l) {
+      if (a.acc == 2) {
+        ob[l] += UNB[l];
+        vb[l] += VNB[l];
+        wb[l] += WNB[l];
+      }
+      au[l] += ob[l] * dtau;
+      av[l] += vb[l] * dtau;
+      if (col.hb) aw[l] += wb[l] * dtau;
+    }
+    stvec<V>(a.Rub, r0 + i0, au);
+    stvec<V>(a.Rvb, r0 + i0, av);
+    stvec<V>(a.Rwb, r0 + i0, aw);
+  }
+#pragma unroll
+  for (int l = 0; l < V; ++l) {
+    at[l] += tb[l];
+    as[l] += sb[l];
+  }
+  stvec<V>(a.trhob, r0 + i0, at);
+  stvec<V>(a.psb, r0 + i0, as);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -939,32 +943,28 @@ __global__ void __launch_bounds__(AB) k_smag_state_vjp(Dims d, Phys ph, Cols c, 
 
 }  // namespace
 
-cudaError_t launch_acoustic_vjp(const Dims& d, const Phys& ph, const Cols& c, const AcousticVjpArgs& a, float dtau,
-                                cudaStream_t st, const cudaAccessPolicyWindow* win) {
-  constexpr int V = ACOUSTIC_VJP_VEC;
-  if (d.nx % V == 0) {
-    // small blocks: many registers per thread (a register cap that made the 4-wide kernel spill
-    // float4 values faulted with a misaligned address)
-    dim3 b(16, 4, 1);
-    dim3 g((d.nx / V + 15) / 16, (d.ny + 3) / 4, d.nz);
-    if (win) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = g;
-      cfg.blockDim = b;
-      cfg.stream = st;
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeAccessPolicyWindow;
-      at[0].val.accessPolicyWindow = *win;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      return cudaLaunchKernelEx(&cfg, k_acoustic_vjpv<V>, d, ph, c, a, dtau);
-    }
-    k_acoustic_vjpv<V><<<g, b, 0, st>>>(d, ph, c, a, dtau);
-    return cudaGetLastError();
+template <int V>
+static cudaError_t launch_vjpv(const Dims& d, const Phys& ph, const Cols& c, const AcousticVjpArgs& a, float dtau,
+                               cudaStream_t st) {
+  // blocks as the forward sub-step's
+  const int nq = d.nx / V;
+  constexpr int kMaxGrid = 65535;
+  constexpr int BXT = V == 1 ? 32 : 16;
+  const bool flat = nq % BXT != 0 || d.ny / (VJP_T / BXT) >= kMaxGrid / 2;
+  const dim3 b = flat ? dim3(VJP_T) : dim3(BXT, VJP_T / BXT);
+  dim3 g = flat ? dim3((nq * d.ny + VJP_T - 1) / VJP_T) : dim3(nq / BXT, (d.ny + b.y - 1) / b.y);
+  for (int k0 = 0; k0 < d.nz; k0 += kMaxGrid) {   // one launch, but for grids of more than 65535 levels
+    g.z = d.nz - k0 < kMaxGrid ? d.nz - k0 : kMaxGrid;
+    k_acoustic_vjpv<V><<<g, b, 0, st>>>(d, ph, c, a, dtau, (int)flat, k0);
   }
-  const unsigned g = (unsigned)((d.cells() + AB - 1) / AB);
-  k_acoustic_vjp<<<g, AB, 0, st>>>(d, ph, c, a, dtau);
   return cudaGetLastError();
+}
+
+cudaError_t launch_acoustic_vjp(const Dims& d, const Phys& ph, const Cols& c, const AcousticVjpArgs& a, float dtau,
+                                cudaStream_t st) {
+  if (d.nx % 4 == 0) return launch_vjpv<4>(d, ph, c, a, dtau, st);
+  if (d.nx % 2 == 0) return launch_vjpv<2>(d, ph, c, a, dtau, st);
+  return launch_vjpv<1>(d, ph, c, a, dtau, st);
 }
 
 cudaError_t launch_stage_pointwise_vjp(const Dims& d, const Phys& ph, const Cols& c, const StageVjpArgs& a,

@@ -12,6 +12,7 @@ struct AcousticVjpArgs {
   const float *unb, *vnb, *wnb, *pnb;    // adjoint of the output
   float *ub, *vb, *wb, *pb;              // adjoint of the input (written)
   float *Rub, *Rvb, *Rwb, *trhob, *psb;  // accumulated
+  int acc;  // to Rub, Rvb, Rwb: 0 nothing, 1 ub, vb, wb, 2 those and unb, vnb, wnb
 };
 
 // Pointwise part of one stage backwards (after its acoustic loop).
@@ -61,7 +62,7 @@ cudaError_t launch_smag_vjp(const Dims&, const Phys&, const Cols&, State x0, con
 
 // win: an L2 access-policy window for the launch (the accumulators)
 cudaError_t launch_acoustic_vjp(const Dims&, const Phys&, const Cols&, const AcousticVjpArgs&, float dtau,
-                                cudaStream_t, const cudaAccessPolicyWindow* win = nullptr);
+                                cudaStream_t);
 cudaError_t launch_stage_pointwise_vjp(const Dims&, const Phys&, const Cols&, const StageVjpArgs&, cudaStream_t);
 // x0b (non-null fields): also x0b += xsb, after the update (the first stage's input is the step's input)
 cudaError_t launch_massdiv_vjp(const Dims&, const Phys&, const Cols&, const float* divb, State xsb, cudaStream_t,

@@ -52,3 +52,27 @@ def test_repeated_reverse_passes_agree(built_lib, dims):
         for _ in range(4):
             same(other, run(0.25))
         same(first, run(0.18))
+
+
+@pytest.mark.parametrize("nx,copies", [(15, 4), (30, 2), (44, 2)], ids=["odd", "even", "four"])
+def test_reverse_pass_on_rows_of_any_length(built_lib, nx, copies):
+    """Periodic copies side by side are the same flow, so a grid of nx points and one of `copies` times as
+    many give the same step and the same adjoint.  The kernels take one, two or four cells a thread by the
+    divisors of nx: the same sums, a contraction apart (100 sub-steps of a few operations at 2^-24: 2e-5)."""
+    torch = pytest.importorskip("torch")
+    from lex_gb300 import autograd as lag
+    ny, nz = 13, 9
+    with _solver(nx, ny, nz) as S, _solver(nx * copies, ny, nz) as D:
+        x0 = lag.get_state(S)
+        g = torch.Generator(device="cpu").manual_seed(2)
+        seeds = [torch.randn(t.shape, generator=g).cuda() for t in x0]
+
+        def run(solver, n):
+            x = [torch.cat([t.detach()] * n, 2).contiguous().requires_grad_(True) for t in x0]
+            y = lag.step(solver, x)
+            return list(y) + list(torch.autograd.grad(y, x, grad_outputs=[torch.cat([t] * n, 2) for t in seeds]))
+        for i, (a, b) in enumerate(zip(run(S, 1), run(D, copies))):
+            a, b = a.detach().double(), b.detach().double()
+            for m in range(copies):
+                part = b[:, :, m * nx:(m + 1) * nx]
+                assert float((part - a).norm()) <= 2e-5 * float(a.norm()), (i, m)

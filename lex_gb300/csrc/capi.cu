@@ -1344,7 +1344,6 @@ int adj_reverse(lexgb_ctx* c, AdjWork& w, const State& x0, int nstages) {
   if (turb) CKS(zero_fields(c, w.sgsb[0], 5));
   for (int s = nstages - 1; s >= 0; --s) {
     const State xs = s == 0 ? A : w.S[s];
-    CKS(zero_fields(c, w.Xs.T, NFIELD));
     CKS(zero_fields(c, w.Rub, 5));
     // acoustic loop backwards
     const float* adj[4] = {w.Cur.u, w.Cur.v, w.Cur.w, w.Cur.p};

@@ -22,7 +22,7 @@ struct StageVjpArgs {
   const float *Tnb, *qnb;                     // adjoint of the stage's theta / qv outputs
   const float *Rub, *Rvb, *Rwb, *trhob, *psb; // from the acoustic loop
   float dts;
-  State xsb;                                  // adjoint of the stage input (accumulated)
+  State xsb;                                  // adjoint of the stage input (written)
   State x0b;                                  // adjoint of the big step's input (T, q accumulated)
   const float* acb[4];                        // adjoint of the acoustic loop's input u, v, w, pi' (added to x0b)
   float* cb[5];                               // adjoint of the flux convergence per field (u, v, w, T, q)

@@ -576,23 +576,29 @@ __global__ void __launch_bounds__(TcLayout<CIN, COUT>::THREADS, 2)
 //   dW[tap][co][ci] += sum over points p of g[p][co] x[p + off(tap)][ci]
 //
 // as D[M][N] += A[M][K] B[K][N] with K = the 128 points of an 8 (x) x 16 (y) tile at one level,
-// N = the gradient's channels co (16 or 32) and M = 128 rows (dy shift s, input channel ci): the
-// rows of A are the input plane read 16 / CG (4 or 8) rows apart, so one MMA covers the y offsets
-// -1, 0, +1 (and spare shifts whose rows are dropped).  Each of the nine (dz, dx) offset pairs has
+// N = the gradient's channels co (16 or 32) at up to three levels and M = 128 rows (dy shift s, input
+// channel ci): the rows of A are the input plane read 16 / CG (4 or 8) rows apart, so one MMA covers the
+// y offsets -1, 0, +1 (and spare shifts whose rows are dropped), and with the gradient planes below, at and
+// above the input plane side by side in B the three z offsets too.  A costs the same however wide N is (its
+// reads from shared memory, about 60 cycles an MMA): with one MMA for each (dz, dx) a level took 72 of
+// them, and 32 -> 32 channels on 128x128x64 127 us; with 24, 62 us.  Each of the nine (dx, dz) pairs has
 // its own accumulator in tensor memory; a block keeps them over all the (tile, level chunk) items
 // it takes and adds them to dW once, at the end.  Both operands are MN-major (the channels are
 // the contiguous 16 bytes of a core matrix; its 8 rows are 8 consecutive points along x):
-//   x planes  Xsm[HY][CG][10][8]   halo rows y0-1 .. y0+14+SH, all channel groups of a row
+//   x planes  Xsm[R][HY][CG][10][8]  halo rows y0-1 .. y0+14+SH, all channel groups of a row
 //                                  together (a 5-D tensor map with the channel group as its own
 //                                  dimension), so the next M block (next channel group, or the
 //                                  next row after the last group) is 160 bytes on (SBO) and the
 //                                  next K block (the next row of the tile) one halo row on (LBO)
-//   gradient  Gsm[NP/8][16][8][8]  next N block = next channel group, 2048 bytes (SBO); next K
-//                                  block = next row, 128 bytes (LBO)
-// Warp 4 loads plane p of x (with its halo; zero outside the grid) and, for the levels of the
-// item, plane p of g into one slot of a ring; warp 5 issues the 72 MMAs of a level (3 dz x 3 dx x
-// 8 pairs of rows); warps 0-3 wait for the last MMA, read their lane quarter of the nine
-// accumulators and add the rows of the y offsets -1..+1 to dW (atomicAdd).
+//   gradient  Gsm[R+2][NP/8][16][8][8]  next N block = next channel group, then the next plane, 2048
+//                                  bytes (SBO); next K block = next row, 128 bytes (LBO).  Planes R, R+1
+//                                  hold planes 0, 1 again, so that three planes in a row are adjacent
+//                                  wherever they begin
+// Step j of an item takes input plane p = z0 - 1 + j.  Warp 4 loads it (with its halo; zero outside the
+// grid) and gradient plane p + 1, where the item has it, into slot j % R; warp 5 issues the 24 MMAs of a
+// step (3 dx x 8 pairs of rows) on gradient planes p - 1 .. p + 1; warps 0-3 clear the accumulators, wait
+// for the last MMA, read their lane quarter of them and add the rows of the y offsets -1..+1 to dW
+// (atomicAdd).
 template <int CG, int NP>
 struct DwLayout {
   static constexpr int SH = 16 / CG;                        // y shifts in the 128 rows of M
@@ -602,13 +608,13 @@ struct DwLayout {
   static constexpr int X_PAD = (X_BYTES + 127) / 128 * 128;
   static constexpr int G_GROUP = TC_TY * TC_TX * 16;        // one 8-channel group of a gradient tile
   static constexpr int G_BYTES = NP / 8 * G_GROUP;
-  static constexpr int SLOT = X_PAD + G_BYTES;
   static constexpr int R = 6;                               // ring slots
+  static constexpr int G_AT = R * X_PAD, BAR_AT = G_AT + (R + 2) * G_BYTES;
   static constexpr int TMEM_COLS = 9 * NP <= 256 ? 256 : 512;
   static constexpr int BAR_BYTES = (2 * R + 1) * 8 + 16;
   // + 4 KB after the barriers: an operand's core matrices, read with the two descriptor strides
   // either way round, stay inside the allocation
-  static constexpr size_t NEED = 128 + (size_t)R * SLOT + BAR_BYTES + 4096;
+  static constexpr size_t NEED = 128 + (size_t)BAR_AT + BAR_BYTES + 4096;
   // at most 512 / TMEM_COLS blocks per SM, so that no block waits for another's tensor memory
   static constexpr size_t FLOOR = TMEM_COLS == 512 ? 120 * 1024 : 80 * 1024;
   static constexpr size_t BYTES = NEED < FLOOR ? FLOOR : NEED;
@@ -633,12 +639,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   extern __shared__ unsigned char tc_raw[];
   const uint32_t raw_s = smem_u32(tc_raw);
   unsigned char* smem = tc_raw + ((128u - (raw_s & 127u)) & 127u);
-  const uint32_t ring_s = smem_u32(smem), bar_s = ring_s + R * L::SLOT;
-  auto slot = [&](long long j) { return ring_s + (uint32_t)(j % R) * L::SLOT; };
-  auto full = [&](long long j) { return bar_s + 8u * (uint32_t)(j % R); };
-  auto empty = [&](long long j) { return bar_s + 8u * (R + (uint32_t)(j % R)); };
+  const uint32_t x_s = smem_u32(smem), g_s = x_s + L::G_AT, bar_s = x_s + L::BAR_AT;
+  auto slot = [&](long long j) { return (uint32_t)(j % R); };
+  auto full = [&](long long j) { return bar_s + 8u * slot(j); };
+  auto empty = [&](long long j) { return bar_s + 8u * (R + slot(j)); };
   const uint32_t done = bar_s + 8u * (2 * R);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + R * L::SLOT + (2 * R + 1) * 8);
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::BAR_AT + (2 * R + 1) * 8);
   volatile int* abort = reinterpret_cast<volatile int*>(tslot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -661,31 +667,41 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tslot;
+  if (warp < 4) {   // warp-aligned lane quarters
+    for (int q = 0; q < 9 * NP / 16; ++q) tmem_zero_cols<16>(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(16 * q));
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
   const int tiles_x = (nx + TC_TX - 1) / TC_TX, tiles_y = (ny + TC_TY - 1) / TC_TY;
   const int chunks = (nz + zc - 1) / zc, items = tiles_x * tiles_y * chunks;
 
   if (warp == 4) {
     // ---------------- producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       long long j = 0;
       bool ok = true;
       for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
         const int x0 = (it % tiles_x) * TC_TX, y0 = ((it / tiles_x) % tiles_y) * TC_TY;
         const int z0 = (it / (tiles_x * tiles_y)) * zc, z1 = min(z0 + zc, nz);
         for (int p = z0 - 1; p <= z1; ++p, ++j) {
-          if (j >= R && !mbar_wait(empty(j), (uint32_t)((j / R - 1) & 1), abort)) {
+          // the slot's gradient plane, loaded at step j - R, is last read at step j - R + 2
+          const long long m = j - R + 2;
+          if (m >= 0 && !mbar_wait(empty(m), (uint32_t)((m / R) & 1), abort)) {
             atomicAdd(&g_tc_timeouts, 1u);
             *abort = 1;
             ok = false;
             break;
           }
-          const bool with_g = p >= z0 && p < z1;
-          mbar_expect_tx(full(j), L::X_BYTES + (with_g ? L::G_BYTES : 0));
-          tma_load_5d(slot(j), &xmap, 0, x0 - 1, 0, y0 - 1, p, full(j));
-          if (with_g)
+          const uint32_t q = slot(j);
+          const int copies = p + 1 < z1 ? (q < 2 ? 2 : 1) : 0;
+          mbar_expect_tx(full(j), L::X_BYTES + copies * L::G_BYTES);
+          tma_load_5d(x_s + q * L::X_PAD, &xmap, 0, x0 - 1, 0, y0 - 1, p, full(j));
+          for (int n = 0; n < copies; ++n)
             for (int cg = 0; cg < NP / 8; ++cg)
-              tma_load_4d(slot(j) + L::X_PAD + cg * L::G_GROUP, &gmap, cg * 8, x0, y0, p, full(j));
+              tma_load_4d(g_s + (q + n * R) * L::G_BYTES + cg * L::G_GROUP, &gmap, cg * 8, x0, y0, p + 1, full(j));
         }
       }
       // the copies this thread issued have landed before the block's memory goes (bounded)
@@ -693,42 +709,36 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     }
   } else if (warp == 5) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = tc_idesc(128, NP) | (1u << 15) | (1u << 16);   // A and B MN-major
+    if (elect_one()) {
       long long j = 0;
-      bool ok = true, first = true;
+      bool ok = true;
       for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
         const int z0 = (it / (tiles_x * tiles_y)) * zc, z1 = min(z0 + zc, nz);
-        const long long jb = j;   // load index of plane z0 - 1
-        for (int z = z0; z < z1 && ok; ++z) {
-          const long long jz = jb + (z - z0);   // plane z - 1; planes z and z + 1 follow
-          for (int q = (z == z0 ? 0 : 2); q <= 2 && ok; ++q) ok = mbar_wait(full(jz + q), (uint32_t)(((jz + q) / R) & 1), abort);
+        const long long jb = j;
+        for (int p = z0 - 1; p <= z1; ++p, ++j) {
+          ok = mbar_wait(full(j), (uint32_t)((j / R) & 1), abort);
           if (!ok) {
             atomicAdd(&g_tc_timeouts, 1u);
             *abort = 1;
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint64_t b0 = smem_desc(slot(jz + 1) + L::X_PAD, 128, L::G_GROUP);
+          // gradient planes p - 1 + n, n0 <= n < n1, of the item; plane z was loaded at step jb + z - z0
+          const int n0 = max(0, z0 + 1 - p), n1 = min(3, z1 + 1 - p);
+          const uint32_t idesc = tc_idesc(128, (n1 - n0) * NP) | (1u << 15) | (1u << 16);   // A and B MN-major
+          const uint64_t a0 = smem_desc(x_s + slot(j) * L::X_PAD, L::ROW_BYTES, TC_HX * 16);
+          const uint64_t b0 = smem_desc(g_s + slot(jb + (p - 1 + n0 - z0)) * L::G_BYTES, 128, L::G_GROUP);
+          const uint32_t col = tmem + (uint32_t)(n0 * NP);
 #pragma unroll
-          for (int dz = 0; dz < 3; ++dz) {
-            const uint64_t a0 = smem_desc(slot(jz + dz), L::ROW_BYTES, TC_HX * 16);
+          for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
-            for (int dx = 0; dx < 3; ++dx)
-#pragma unroll
-              for (int m = 0; m < 8; ++m) {
-                const uint64_t ad = a0 + (uint64_t)((2 * m * L::ROW_BYTES + dx * 16) >> 4);
-                const uint64_t bd = b0 + (uint64_t)((2 * m * 128) >> 4);
-                mma_bf16_tc(tmem + (uint32_t)((dz * 3 + dx) * NP), ad, bd, idesc, (first && m == 0) ? 0u : 1u);
-              }
-          }
-          first = false;
-          mma_commit(empty(jz));   // plane z - 1 is not read again
+            for (int m = 0; m < 8; ++m) {
+              const uint64_t ad = a0 + (uint64_t)((2 * m * L::ROW_BYTES + dx * 16) >> 4);
+              const uint64_t bd = b0 + (uint64_t)((2 * m * 128) >> 4);
+              mma_bf16_tc(col + (uint32_t)(dx * 3 * NP), ad, bd, idesc, 1u);
+            }
+          mma_commit(empty(j));
         }
-        if (!ok) break;
-        mma_commit(empty(jb + (z1 - z0)));       // planes z1 - 1 and z1
-        mma_commit(empty(jb + (z1 - z0) + 1));
-        j = jb + (z1 - z0) + 2;
       }
       mma_commit(done);
       mbar_wait_long(done, 0, nullptr);   // the MMAs are complete before the tensor memory goes
@@ -747,7 +757,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         for (int c = 0; c < NP; c += 16) tmem_load16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(acc * NP + c), v + c);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (mine) {
-          const int tap = (acc / 3) * 9 + s * 3 + acc % 3;
+          const int tap = (2 - acc % 3) * 9 + s * 3 + acc / 3;   // gradient plane n of a step: dz = 2 - n
           float* d = dw + (long long)tap * cout * cin + ci;
 #pragma unroll
           for (int co = 0; co < NP; ++co)
@@ -936,14 +946,14 @@ cudaError_t launch_dw(int nx, int ny, int nz, int cin, int cout, const void* x, 
   if (!make_dw_xmap(&xmap, x, nx, ny, nz, cin, L::HY) || !make_dw_gmap(&gmap, g, nx, ny, nz, NP))
     return cudaErrorInvalidValue;
   // level chunks: the count that ends soonest when every block takes ceil(items / blocks) items
-  // of chunk + 1 plane times (ties: fewer items, each of which loads two extra planes)
+  // of chunk + 2 steps (ties: fewer items)
   const long long tiles = (long long)((nx + TC_TX - 1) / TC_TX) * ((ny + TC_TY - 1) / TC_TY);
   int zc = nz;
   long long best = -1;
   for (int nch = 1; nch <= nz; ++nch) {
     const int z = (nz + nch - 1) / nch;
     const long long items = tiles * ((nz + z - 1) / z), blocks = items < cap ? items : cap;
-    const long long cost = (items + blocks - 1) / blocks * (z + 1);
+    const long long cost = (items + blocks - 1) / blocks * (z + 2);
     if (best < 0 || cost < best) {
       best = cost;
       zc = z;

@@ -79,6 +79,40 @@ def test_convolution_at_the_edges_of_its_tiles(kernel, name, dims, cin, cout, sh
         assert bool(buf[:lo].isnan().all()) and bool(buf[lo + n * cout:].isnan().all())
 
 
+# one level, two; a plane ring that goes round (and whose first planes are held twice) within an item and
+# over several items of a block; tiles that the grid does not fill
+DW_DIMS = [(8, 16, 1), (8, 16, 2), (8, 16, 7), (16, 16, 150), (64, 48, 61), (20, 13, 23)]
+
+
+@pytest.mark.parametrize("cin,cout,gstride", [(32, 32, 32), (16, 32, 32), (32, 8, 16)])
+@pytest.mark.parametrize("dims", DW_DIMS, ids=str)
+def test_weight_gradient_at_the_edges_of_its_chunks(kernel, dims, cin, cout, gstride):
+    """Against the FP64 sums of the same BF16 products: at most 2 npts additions in FP32, in any order and with
+    truncation, are within npts 2^-22 of the sum of their magnitudes."""
+    torch = pytest.importorskip("torch")
+    from lex_gb300 import sgs_cnn
+    lib = kernel("tcgen05")
+    nx, ny, nz = dims
+    n = nx * ny * nz
+    gen = torch.Generator(device="cpu").manual_seed(n + cin)
+    x = torch.randn(n, cin, generator=gen).cuda().bfloat16()
+    g = torch.randn(n, gstride, generator=gen).cuda().bfloat16()
+    dw = torch.zeros(27, cout, cin, device="cuda")
+    p = sgs_cnn._p
+    assert lib.lexgb_cnn_conv3d_dw(nx, ny, nz, cin, cout, gstride, p(x), p(g), p(dw), None, sgs_cnn._stream()) == 0
+    torch.cuda.synchronize()
+
+    def sums(x, g):
+        xp = torch.zeros(nz + 2, ny + 2, nx + 2, cin, device="cuda", dtype=torch.float64)
+        xp[1:-1, 1:-1, 1:-1] = x.double().reshape(nz, ny, nx, cin)
+        gd = g.double()[:, :cout].reshape(nz, ny, nx, cout)
+        return torch.stack([torch.einsum("zyxo,zyxi->oi", gd, xp[a:a + nz, b:b + ny, c:c + nx])
+                            for a in range(3) for b in range(3) for c in range(3)])
+    ref, mag = sums(x, g), sums(x.abs(), g.abs())
+    assert bool(((dw.double() - ref).abs() <= n * 2.0 ** -22 * mag).all())
+    assert float((dw.double() - ref).norm()) <= 1e-5 * float(ref.norm())   # as the kernel's own tests
+
+
 @pytest.mark.parametrize("dims", [(16, 5, 3), (32, 21, 33), (64, 64, 65)], ids=str)
 def test_network_and_gradients_at_the_edges(built_lib, dims):
     """The whole network and its gradients against PyTorch, at the BF16 level of the kernels' own tests."""

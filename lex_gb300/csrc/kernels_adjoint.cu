@@ -646,6 +646,93 @@ __global__ void __launch_bounds__(AB) k_adv_face_vjp(Dims d, Phys ph, Cols c, Ad
   a.mb[3][id] = mbar_s;
 }
 
+// Directions y and z (D = 1, 2) of the flux adjoints in one pass: a thread walks a chunk of a column along D
+// for one field, with the six points of the stencil and the six adjoints that still receive slots in
+// registers, so the slots are never stored (34 fields a direction written and read back otherwise:
+// 192x192x96 320 us a direction and stage with the gather, now 245; 64x64x64 29.5, now 28).  Bound by the WENO derivatives' arithmetic
+// (about 350 instructions a face).  A chunk of n points takes n + 5 faces.  The mass-flux adjoints of u, v, w
+// and theta go to mb, qv's to P[0][0].
+constexpr int MARCH_T = 128;
+template <int D>
+__global__ void __launch_bounds__(MARCH_T) k_adv_march_vjp(Dims d, Phys ph, Cols c, AdvVjpArgs a, int chunk) {
+  const int nx = d.nx, ny = d.ny, nz = d.nz, plane = d.plane();
+  const int f = blockIdx.z;
+  const unsigned col = blockIdx.x * MARCH_T + threadIdx.x;
+  if (col >= (unsigned)(D == 1 ? nx * nz : plane)) return;
+  const int i = (int)(col % nx), r = (int)(col / nx);   // r: level (y) or row (z)
+  if (D == 1 && f == 2 && r == 0) return;               // w = 0 on the ground
+  const int n = D == 1 ? ny : (f == 2 ? nz + 1 : nz), stride = D == 1 ? nx : plane;
+  const int base = D == 1 ? r * plane + i : r * nx + i;
+  const int p0 = blockIdx.y * chunk, p1 = min(p0 + chunk, n);
+  if (p0 >= p1) return;
+  const float* const phi = a.phi[f];
+  const float* const cb = a.cb[f];
+  const float* const wind = D == 1 ? a.xs.v : a.xs.w;
+  float* const out = f == 0 ? a.xsb.u : f == 1 ? a.xsb.v : f == 2 ? a.xsb.w : f == 3 ? a.xsb.T : a.xsb.q;
+  float* const mb = f < 4 ? a.mb[f] : a.P[0][0];
+  const float rd = D == 1 ? ph.rdy : ph.rdz, eps = f < 3 ? kWepsMom : (f == 3 ? kWepsTheta : kWepsQv);
+  // rows -5 .. ny + 4 of at least four
+  auto at = [&](int p) { return base + (D == 1 ? wrapx(wrapx(p, ny), ny) : p) * stride; };
+  auto inside = [&](int p) { return D == 1 || (p >= 0 && p < n); };
+  // the two winds of a face's mass flux (the same one for theta and qv) and their factors
+  const int da = f == 0 ? wrapx(i - 1, nx) - i : D == 2 && f == 1 ? (wrapx(r - 1, ny) - r) * nx : D == 1 && f == 2 ? -plane : 0;
+  const int ha = f == D ? 1 : 0;   // the wind's own field: the points on either side of the face
+  const float half = f < 3 ? 0.5f : 0.f;
+  float w1 = f < 3 ? 0.5f : 1.f, w0 = half;
+  if (D == 1) {
+    w0 *= f == 2 ? c.rho[r - 1] : c.rho[r];
+    w1 *= c.rho[r];
+  }
+  // faces p0 - 2 .. p1 + 2 touch the chunk's points
+  float s[6], acc[6];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    acc[q] = 0.f;
+    s[q] = q > 0 && inside(p0 - 6 + q) ? LD(phi, at(p0 - 6 + q)) : 0.f;   // points H - 4 .. H + 1 of the first face
+  }
+  float cbm = inside(p0 - 3) ? LD(cb, at(p0 - 3)) : 0.f;
+  float nphi, ncb, nwa, nw, nout;
+  auto load = [&](int H) {   // what face H adds to the window
+    const bool face = D == 1 || (H >= 1 && H < n);
+    nphi = inside(H + 2) ? LD(phi, at(H + 2)) : 0.f;
+    ncb = inside(H) ? LD(cb, at(H)) : 0.f;
+    nw = face ? LD(wind, at(H)) : 0.f;
+    nwa = face && f < 3 ? LD(wind, at(H - ha) + da) : 0.f;
+    nout = H - 3 >= p0 ? out[at(H - 3)] : 0.f;
+  };
+  load(p0 - 2);
+#pragma unroll 1
+  for (int H = p0 - 2; H <= p1 + 2; ++H) {
+#pragma unroll
+    for (int q = 0; q < 5; ++q) s[q] = s[q + 1];
+    s[5] = nphi;
+    const float cbp = ncb, wa = nwa, wp = nw, o = nout;
+    if (H < p1 + 2) load(H + 1);
+    if (D == 1 || (H >= 1 && H < n)) {
+      float m;
+      if (D == 1)
+        m = w0 * wa + w1 * wp;
+      else if (f == 2)
+        m = 0.5f * (wa + wp) * c.rho[H - 1];
+      else
+        m = (w0 * wa + w1 * wp) * c.rho_face[H];
+      const float Fb = (cbp - cbm) * rd;
+      float g[6];
+      const float W = D == 1 ? lateral_grad(m, s, eps, g) : vertical_grad(m, s, H, n, eps, g);
+      const float fm = Fb * m;
+#pragma unroll
+      for (int q = 0; q < 6; ++q) acc[q] += fm * g[q];
+      if (H >= p0 && H < p1) mb[at(H)] = Fb * W;
+    }
+    cbm = cbp;
+    if (H - 3 >= p0) out[at(H - 3)] = o + acc[0];
+#pragma unroll
+    for (int q = 0; q < 5; ++q) acc[q] = acc[q + 1];
+    acc[5] = 0.f;
+  }
+}
+
+// D = 0: the slots into the fields; every D: the mass-flux adjoints into the wind of that direction
 template <int D>
 __global__ void __launch_bounds__(AB) k_adv_gather_vjp(Dims d, Phys ph, Cols c, AdvVjpArgs a) {
   const unsigned t = blockIdx.x * AB + threadIdx.x;
@@ -653,17 +740,16 @@ __global__ void __launch_bounds__(AB) k_adv_gather_vjp(Dims d, Phys ph, Cols c, 
   if (t >= d.faces()) return;
   const int i = (int)(t % nx), j = (int)((t / nx) % ny), k = (int)(t / plane);
   const int id = (int)t;
-  float* out[5] = {a.xsb.u, a.xsb.v, a.xsb.w, a.xsb.T, a.xsb.q};
-  for (int f = 0; f < 5; ++f) {
-    const int n = f == 2 ? nz + 1 : nz;
-    if (k >= n) continue;
-    float acc = 0.f;
-    // the flux at point p+3-q names this point in its slot q
-    for (int q = 0; q < 6; ++q) {
-      const int pf = along<D>(d, i, j, k, 3 - q, nz + 1);  // fluxes exist on face levels 0..nz
-      if (pf >= 0) acc += LD(a.P[f][q], pf);
+  if constexpr (D == 0) {
+    float* out[5] = {a.xsb.u, a.xsb.v, a.xsb.w, a.xsb.T, a.xsb.q};
+    for (int f = 0; f < 5; ++f) {
+      const int n = f == 2 ? nz + 1 : nz;
+      if (k >= n) continue;
+      float acc = 0.f;
+      // the flux at point p+3-q names this point in its slot q
+      for (int q = 0; q < 6; ++q) acc += LD(a.P[f][q], along<D>(d, i, j, k, 3 - q, nz + 1));
+      out[f][id] += acc;
     }
-    out[f][id] += acc;
   }
   // mass-flux adjoints into the wind of direction D
   const int ip = wrapx(i + 1, nx), jp = wrapx(j + 1, ny);
@@ -680,7 +766,7 @@ __global__ void __launch_bounds__(AB) k_adv_gather_vjp(Dims d, Phys ph, Cols c, 
     if (k >= nz) return;
     const float r = c.rho[k];
     const int row = k * plane;
-    float vb = r * LD(a.mb[3], id);
+    float vb = r * (LD(a.mb[3], id) + LD(a.P[0][0], id));
     vb += 0.5f * r * (LD(a.mb[0], id) + LD(a.mb[0], row + j * nx + ip));
     vb += 0.5f * r * (LD(a.mb[1], id) + LD(a.mb[1], row + jp * nx + i));
     vb += 0.5f * r * ((k >= 1 ? LD(a.mb[2], id) : 0.f) + (k + 1 < nz ? LD(a.mb[2], id + plane) : 0.f));
@@ -690,7 +776,7 @@ __global__ void __launch_bounds__(AB) k_adv_gather_vjp(Dims d, Phys ph, Cols c, 
     float wb = 0.f;
     if (k >= 1 && k < nz) {
       const float rf = c.rho_face[k];
-      wb += rf * LD(a.mb[3], id);
+      wb += rf * (LD(a.mb[3], id) + LD(a.P[0][0], id));
       wb += 0.5f * rf * (LD(a.mb[0], id) + LD(a.mb[0], row + j * nx + ip));
       wb += 0.5f * rf * (LD(a.mb[1], id) + LD(a.mb[1], row + jp * nx + i));
     }
@@ -1037,13 +1123,33 @@ cudaError_t launch_smag_vjp(const Dims& d, const Phys& ph, const Cols& c, State 
   return cudaGetLastError();
 }
 
+// Chunks of a column: ten blocks an SM, and at least 16 points, of which a chunk takes 21 faces (64x64x64, two
+// steps and their reverse pass, 1, 2, 4, 8 chunks: 3.20, 3.05, 3.03, 3.08 ms; 192x192x96, one step, 1, 2, 3, 8:
+// 9.54, 9.44, 9.44, 9.60)
+template <int D>
+static cudaError_t launch_march(const Dims& d, const Phys& ph, const Cols& c, const AdvVjpArgs& a, cudaStream_t st) {
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  const int n = D == 1 ? d.ny : d.nz + 1;
+  const long long cols = ((long long)(D == 1 ? d.nx * d.nz : d.plane()) + MARCH_T - 1) / MARCH_T;
+  const long long want = (10LL * sms + 5 * cols - 1) / (5 * cols), most = n / 16 > 1 ? n / 16 : 1;
+  const int chunk = (int)((n + (want < most ? want : most) - 1) / (want < most ? want : most));
+  const unsigned count = (unsigned)((n + chunk - 1) / chunk);
+  k_adv_march_vjp<D><<<dim3((unsigned)cols, count, 5), MARCH_T, 0, st>>>(d, ph, c, a, chunk);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_adv_vjp(const Dims& d, const Phys& ph, const Cols& c, const AdvVjpArgs& a, cudaStream_t st) {
   const unsigned g = (unsigned)((d.faces() + AB - 1) / AB);
   k_adv_face_vjp<0><<<g, AB, 0, st>>>(d, ph, c, a);
   k_adv_gather_vjp<0><<<g, AB, 0, st>>>(d, ph, c, a);
-  k_adv_face_vjp<1><<<g, AB, 0, st>>>(d, ph, c, a);
+  cudaError_t e = launch_march<1>(d, ph, c, a, st);
+  if (e != cudaSuccess) return e;
   k_adv_gather_vjp<1><<<g, AB, 0, st>>>(d, ph, c, a);
-  k_adv_face_vjp<2><<<g, AB, 0, st>>>(d, ph, c, a);
+  e = launch_march<2>(d, ph, c, a, st);
+  if (e != cudaSuccess) return e;
   k_adv_gather_vjp<2><<<g, AB, 0, st>>>(d, ph, c, a);
   return cudaGetLastError();
 }

@@ -54,25 +54,28 @@ def test_repeated_reverse_passes_agree(built_lib, dims):
         same(first, run(0.18))
 
 
-@pytest.mark.parametrize("nx,copies", [(15, 4), (30, 2), (44, 2)], ids=["odd", "even", "four"])
-def test_reverse_pass_on_rows_of_any_length(built_lib, nx, copies):
-    """Periodic copies side by side are the same flow, so a grid of nx points and one of `copies` times as
-    many give the same step and the same adjoint.  The kernels take one, two or four cells a thread by the
-    divisors of nx: the same sums, a contraction apart (100 sub-steps of a few operations at 2^-24: 2e-5)."""
+@pytest.mark.parametrize("nx,ny,nz,copies,axis", [(15, 13, 9, 4, 2), (30, 13, 9, 2, 2), (44, 13, 9, 2, 2),
+                                                  (16, 4, 6, 9, 1), (12, 5, 33, 10, 1)],
+                         ids=["odd rows", "even rows", "rows of four", "four rows", "five rows, high"])
+def test_reverse_pass_on_periodic_copies(built_lib, nx, ny, nz, copies, axis):
+    """Periodic copies side by side are the same flow, so a grid and one of `copies` times as many points in x
+    or y give the same step and the same adjoint.  The kernels take one, two or four cells a thread by the
+    divisors of nx, and the flux adjoints walk rows and columns in chunks by their length: the same sums, a
+    contraction or an order apart (100 sub-steps of a few operations at 2^-24: 2e-5)."""
     torch = pytest.importorskip("torch")
     from lex_gb300 import autograd as lag
-    ny, nz = 13, 9
-    with _solver(nx, ny, nz) as S, _solver(nx * copies, ny, nz) as D:
+    n = (nx, ny, nz)
+    big = (nx * copies, ny, nz) if axis == 2 else (nx, ny * copies, nz)
+    with _solver(*n) as S, _solver(*big) as D:
         x0 = lag.get_state(S)
         g = torch.Generator(device="cpu").manual_seed(2)
         seeds = [torch.randn(t.shape, generator=g).cuda() for t in x0]
 
-        def run(solver, n):
-            x = [torch.cat([t.detach()] * n, 2).contiguous().requires_grad_(True) for t in x0]
+        def run(solver, m):
+            x = [torch.cat([t.detach()] * m, axis).contiguous().requires_grad_(True) for t in x0]
             y = lag.step(solver, x)
-            return list(y) + list(torch.autograd.grad(y, x, grad_outputs=[torch.cat([t] * n, 2) for t in seeds]))
+            return list(y) + list(torch.autograd.grad(y, x, grad_outputs=[torch.cat([t] * m, axis) for t in seeds]))
         for i, (a, b) in enumerate(zip(run(S, 1), run(D, copies))):
             a, b = a.detach().double(), b.detach().double()
-            for m in range(copies):
-                part = b[:, :, m * nx:(m + 1) * nx]
-                assert float((part - a).norm()) <= 2e-5 * float(a.norm()), (i, m)
+            for part in torch.split(b, n[2 - axis], axis):
+                assert float((part - a).norm()) <= 2e-5 * float(a.norm()), i

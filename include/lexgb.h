@@ -222,7 +222,7 @@ int lexgb_get_state_interior(lexgb_ctx *ctx, float *fields[6], int on_device);
  * writes xbar, the adjoint of the resident state.  The resident state is not modified.  The
  * forward stages are recomputed internally and every intermediate the reverse pass needs (stage
  * states, divergence, theta_rho, slow tendencies and all acoustic sub-step states) is kept in a
- * workspace allocated on first use (about 110 + 4 * (acoustic sub-steps per step) fields).
+ * workspace allocated on first use (about 100 + 4 * (acoustic sub-steps per step) fields).
  * Arrays are interior-only in the device layout, x fastest: theta, u, v, pi', qv [nz][ny][nx],
  * w [nz+1][ny][nx] (u on west faces, v on south faces, w on faces 0..nz), FP32, host pointers
  * (on_device = 0) or device pointers (on_device = 1).

@@ -1153,14 +1153,13 @@ struct AdjWork {
   float *Rub, *Rvb, *Rwb, *trhob, *psb;
   float* cb[5];
   float* divb;
-  float* P[5][6];
-  float* mb[4];
+  float* mb[5];
   float* sgsb[5];
   SmagLin sl;
   SmagVjpArgs sv;
 };
 
-int adj_fields(const StagePlan& p) { return 6 + 15 + 4 * (p.n[0] + p.n[1] + p.n[2]) + 18 + 8 + 5 + 6 + 34 + 5 + 22 + 6 + 1; }
+int adj_fields(const StagePlan& p) { return 6 + 15 + 4 * (p.n[0] + p.n[1] + p.n[2]) + 18 + 8 + 5 + 6 + 5 + 5 + 22 + 6 + 1; }
 
 int ensure_adjoint(lexgb_ctx* c, AdjWork& w) {
   const StagePlan p = plan_of(c->cfg);
@@ -1193,8 +1192,7 @@ int ensure_adjoint(lexgb_ctx* c, AdjWork& w) {
   w.Rub = take(); w.Rvb = take(); w.Rwb = take(); w.trhob = take(); w.psb = take();
   for (int f = 0; f < 5; ++f) w.cb[f] = take();
   w.divb = take();
-  for (int f = 0; f < 5; ++f) for (int s = 0; s < 6; ++s) w.P[f][s] = take();
-  for (int f = 0; f < 4; ++f) w.mb[f] = take();
+  for (int f = 0; f < 5; ++f) w.mb[f] = take();
   for (int f = 0; f < 5; ++f) w.sgsb[f] = take();
   for (int f = 0; f < 6; ++f) w.sl.s[f] = take();
   w.sl.km = take();
@@ -1379,9 +1377,8 @@ int adj_reverse(lexgb_ctx* c, AdjWork& w, const State& x0, int nstages) {
     aa.phi[0] = xs.u; aa.phi[1] = xs.v; aa.phi[2] = xs.w; aa.phi[3] = xs.T; aa.phi[4] = xs.q;
     for (int f = 0; f < 5; ++f) {
       aa.cb[f] = w.cb[f];
-      for (int q = 0; q < 6; ++q) aa.P[f][q] = w.P[f][q];
+      aa.mb[f] = w.mb[f];
     }
-    for (int f = 0; f < 4; ++f) aa.mb[f] = w.mb[f];
     aa.xsb = w.Xs;
     CK(launch_adv_vjp(d, c->ph, c->cols, aa, c->stream));
     // the first stage's input is the big step's input: its adjoint goes to Xb0 in the same pass

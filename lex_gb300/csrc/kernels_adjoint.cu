@@ -571,87 +571,84 @@ __global__ void __launch_bounds__(AB) k_massdiv_vjp(Dims d, Phys ph, Cols c, con
 // ---------------------------------------------------------------------------------------------
 // WENO advection adjoint, one direction
 // ---------------------------------------------------------------------------------------------
-// point p of field f along direction D: neighbour at offset o (wrapped / or -1 outside the column)
-template <int D>
-__device__ __forceinline__ int along(const Dims& d, int i, int j, int k, int o, int n) {
-  if (D == 0) return (k * d.ny + j) * d.nx + wrapx(i + o, d.nx);
-  if (D == 1) return (k * d.ny + wrapx(j + o, d.ny)) * d.nx + i;
-  const int kk = k + o;
-  return (kk < 0 || kk >= n) ? -1 : (kk * d.ny + j) * d.nx + i;
-}
+// Flux adjoints of a direction, fields 0 u, 1 v, 2 w, 3 theta, 4 qv: the flux between points p-1 and p names the
+// six points p-3 .. p+2 in its slots, and each point adds up the slots that name it; the adjoint of a face's
+// mass flux goes to mb[f].  No slot is stored: 30 fields a direction written and read back otherwise.
 
-// fields: 0 u, 1 v, 2 w, 3 theta, 4 qv
-template <int D>
-__global__ void __launch_bounds__(AB) k_adv_face_vjp(Dims d, Phys ph, Cols c, AdvVjpArgs a) {
-  const unsigned t = blockIdx.x * AB + threadIdx.x;
+// Direction x: a block takes whole rows (nx <= ROW_T) or a segment of one with the five faces beside it, a
+// thread a face, field after field, and the slots meet in shared memory.  Bound by the WENO derivatives'
+// arithmetic (about 350 instructions a face): 192x192x96 315 us a stage with the slots in memory and gathered
+// by another kernel, now 298; 64x64x64 28.4, now 25.9 (with the mass-flux part).  A field a block: 320.
+constexpr int ROW_T = 256;
+__global__ void __launch_bounds__(ROW_T) k_adv_row_vjp(Dims d, Phys ph, Cols c, AdvVjpArgs a, int rows) {
+  __shared__ float slots[2][6][ROW_T];   // two fields' in turn: one barrier a field
   const int nx = d.nx, ny = d.ny, nz = d.nz, plane = d.plane();
-  if (t >= d.faces()) return;
-  const int i = (int)(t % nx), j = (int)((t / nx) % ny), k = (int)(t / plane);
-  const int id = (int)t;
-  const float rd = D == 0 ? ph.rdx : (D == 1 ? ph.rdy : ph.rdz);
-  const int im = wrapx(i - 1, nx), jm = wrapx(j - 1, ny);
-  float mbar_s = 0.f;
-  for (int f = 0; f < 5; ++f) {
-    const int n = f == 2 ? nz + 1 : nz;  // points in the field's column
-    const float* phi = a.phi[f];
-    float slots[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    float mbar = 0.f;
-    bool valid;
-    if (D < 2)
-      valid = f == 2 ? (k >= 1 && k < nz) : (k < nz);
-    else
-      valid = k >= 1 && k < n;  // face H = k between column entries k-1 and k
-    if (valid) {
-      // mass flux
-      float m;
-      const float r = k < nz ? c.rho[k] : 0.f, rm = k >= 1 ? c.rho[k - 1] : 0.f;
-      if (D == 0) {
-        const float* u = a.xs.u;
-        if (f == 0) m = 0.5f * (LD(u, (k * ny + j) * nx + im) + LD(u, id)) * r;
-        else if (f == 1) m = 0.5f * (r * LD(u, (k * ny + jm) * nx + i) + r * LD(u, id));
-        else if (f == 2) m = 0.5f * (rm * LD(u, id - plane) + r * LD(u, id));
-        else m = r * LD(u, id);
-      } else if (D == 1) {
-        const float* v = a.xs.v;
-        if (f == 0) m = 0.5f * (r * LD(v, (k * ny + j) * nx + im) + r * LD(v, id));
-        else if (f == 1) m = 0.5f * (LD(v, (k * ny + jm) * nx + i) + LD(v, id)) * r;
-        else if (f == 2) m = 0.5f * (rm * LD(v, id - plane) + r * LD(v, id));
-        else m = r * LD(v, id);
-      } else {
-        const float* w = a.xs.w;
-        const float rf = c.rho_face[k];
-        if (f == 0) m = 0.5f * (rf * LD(w, (k * ny + j) * nx + im) + rf * LD(w, id));
-        else if (f == 1) m = 0.5f * (rf * LD(w, (k * ny + jm) * nx + i) + rf * LD(w, id));
-        else if (f == 2) m = 0.5f * (LD(w, id - plane) + LD(w, id)) * rm;
-        else m = rf * LD(w, id);
-      }
-      // flux adjoint: the flux between points p-1 and p leaves p-1 and enters p
-      const int pm = along<D>(d, i, j, k, -1, n);
-      const float Fb = (LD(a.cb[f], id) - LD(a.cb[f], pm)) * rd;
-      float s[6];
-      for (int q = 0; q < 6; ++q) {
-        const int pq = along<D>(d, i, j, k, q - 3, n);
-        s[q] = pq >= 0 ? LD(phi, pq) : 0.f;
-      }
-      const float eps = f < 3 ? kWepsMom : (f == 3 ? kWepsTheta : kWepsQv);
-      float g[6];
-      const float W = D < 2 ? lateral_grad(m, s, eps, g) : vertical_grad(m, s, k, n, eps, g);
-      for (int q = 0; q < 6; ++q) slots[q] = Fb * m * g[q];
-      mbar = Fb * W;
-    }
-    for (int q = 0; q < 6; ++q) a.P[f][q][id] = slots[q];
-    if (f < 3) a.mb[f][id] = mbar;
-    else mbar_s += mbar;
+  const int t = threadIdx.x;
+  // the thread's face: row r = (k, j), column i; lo: the row's first slot; own: the face, and the point on its
+  // right, are the block's to store
+  int r, i, lo;
+  bool own, live;
+  if (rows > 0) {
+    r = (int)blockIdx.x * rows + t / nx;
+    i = t % nx;
+    lo = t - i;
+    live = own = t < rows * nx && r < ny * (nz + 1);
+  } else {
+    const int x0 = (int)blockIdx.y * (ROW_T - 5), np = min(ROW_T - 5, nx - x0);
+    r = (int)blockIdx.x;
+    i = wrapx(x0 - 2 + t, nx);
+    lo = 0;
+    live = t < np + 5;
+    own = t >= 2 && t < np + 2;
   }
-  a.mb[3][id] = mbar_s;
+  const int j = r % ny, k = r / ny, row = k * plane + j * nx, id = row + i, im = row + wrapx(i - 1, nx);
+  const bool cell = live && k < nz;
+  int at[6], from[6];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    at[q] = row + wrapx(i + q - 3, nx);
+    from[q] = rows > 0 ? lo + wrapx(i + 3 - q, nx) : t + 3 - q;   // the flux at point p+3-q names p in its slot q
+  }
+  const float* const u = a.xs.u;
+  const float rk = cell ? c.rho[k] : 0.f, u0 = cell ? LD(u, id) : 0.f;
+#pragma unroll 1
+  for (int f = 0; f < 5; ++f) {
+    float* const out = f == 0 ? a.xsb.u : f == 1 ? a.xsb.v : f == 2 ? a.xsb.w : f == 3 ? a.xsb.T : a.xsb.q;
+    const bool mine = own && k < nz + (f == 2);
+    const float o = mine ? out[id] : 0.f;
+    float sl[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (cell && (f != 2 || k >= 1)) {
+      float m = rk * u0;
+      if (f == 0)
+        m = 0.5f * (LD(u, im) + u0) * rk;
+      else if (f == 1)
+        m = 0.5f * (rk * LD(u, k * plane + wrapx(j - 1, ny) * nx + i) + m);
+      else if (f == 2)
+        m = 0.5f * (c.rho[k - 1] * LD(u, id - plane) + m);
+      const float Fb = (LD(a.cb[f], id) - LD(a.cb[f], im)) * ph.rdx;
+      float s[6], g[6];
+#pragma unroll
+      for (int q = 0; q < 6; ++q) s[q] = LD(a.phi[f], at[q]);
+      const float W = lateral_grad(m, s, f < 3 ? kWepsMom : (f == 3 ? kWepsTheta : kWepsQv), g);
+#pragma unroll
+      for (int q = 0; q < 6; ++q) sl[q] = Fb * m * g[q];
+      if (own) a.mb[f][id] = Fb * W;
+    }
+#pragma unroll
+    for (int q = 0; q < 6; ++q) slots[f & 1][q][t] = sl[q];
+    __syncthreads();
+    if (!mine) continue;
+    float acc = 0.f;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) acc += slots[f & 1][q][from[q]];
+    out[id] = o + acc;
+  }
 }
 
 // Directions y and z (D = 1, 2) of the flux adjoints in one pass: a thread walks a chunk of a column along D
 // for one field, with the six points of the stencil and the six adjoints that still receive slots in
-// registers, so the slots are never stored (34 fields a direction written and read back otherwise:
-// 192x192x96 320 us a direction and stage with the gather, now 245; 64x64x64 29.5, now 28).  Bound by the WENO derivatives' arithmetic
-// (about 350 instructions a face).  A chunk of n points takes n + 5 faces.  The mass-flux adjoints of u, v, w
-// and theta go to mb, qv's to P[0][0].
+// registers: 192x192x96 320 us a direction and stage with the slots in memory, now 245; 64x64x64 29.5, now 28.
+// Bound like the rows.  A chunk of n points takes n + 5 faces.
 constexpr int MARCH_T = 128;
 template <int D>
 __global__ void __launch_bounds__(MARCH_T) k_adv_march_vjp(Dims d, Phys ph, Cols c, AdvVjpArgs a, int chunk) {
@@ -669,7 +666,7 @@ __global__ void __launch_bounds__(MARCH_T) k_adv_march_vjp(Dims d, Phys ph, Cols
   const float* const cb = a.cb[f];
   const float* const wind = D == 1 ? a.xs.v : a.xs.w;
   float* const out = f == 0 ? a.xsb.u : f == 1 ? a.xsb.v : f == 2 ? a.xsb.w : f == 3 ? a.xsb.T : a.xsb.q;
-  float* const mb = f < 4 ? a.mb[f] : a.P[0][0];
+  float* const mb = a.mb[f];
   const float rd = D == 1 ? ph.rdy : ph.rdz, eps = f < 3 ? kWepsMom : (f == 3 ? kWepsTheta : kWepsQv);
   // rows -5 .. ny + 4 of at least four
   auto at = [&](int p) { return base + (D == 1 ? wrapx(wrapx(p, ny), ny) : p) * stride; };
@@ -732,32 +729,20 @@ __global__ void __launch_bounds__(MARCH_T) k_adv_march_vjp(Dims d, Phys ph, Cols
   }
 }
 
-// D = 0: the slots into the fields; every D: the mass-flux adjoints into the wind of that direction
+// The mass-flux adjoints of direction D into its wind
 template <int D>
-__global__ void __launch_bounds__(AB) k_adv_gather_vjp(Dims d, Phys ph, Cols c, AdvVjpArgs a) {
+__global__ void __launch_bounds__(AB) k_adv_mass_vjp(Dims d, Phys ph, Cols c, AdvVjpArgs a) {
   const unsigned t = blockIdx.x * AB + threadIdx.x;
   const int nx = d.nx, ny = d.ny, nz = d.nz, plane = d.plane();
   if (t >= d.faces()) return;
   const int i = (int)(t % nx), j = (int)((t / nx) % ny), k = (int)(t / plane);
   const int id = (int)t;
-  if constexpr (D == 0) {
-    float* out[5] = {a.xsb.u, a.xsb.v, a.xsb.w, a.xsb.T, a.xsb.q};
-    for (int f = 0; f < 5; ++f) {
-      const int n = f == 2 ? nz + 1 : nz;
-      if (k >= n) continue;
-      float acc = 0.f;
-      // the flux at point p+3-q names this point in its slot q
-      for (int q = 0; q < 6; ++q) acc += LD(a.P[f][q], along<D>(d, i, j, k, 3 - q, nz + 1));
-      out[f][id] += acc;
-    }
-  }
-  // mass-flux adjoints into the wind of direction D
   const int ip = wrapx(i + 1, nx), jp = wrapx(j + 1, ny);
   if (D == 0) {
     if (k >= nz) return;
     const float r = c.rho[k];
     const int row = k * plane;
-    float ub = r * LD(a.mb[3], id);                                                     // theta, qv
+    float ub = r * (LD(a.mb[3], id) + LD(a.mb[4], id));                                                     // theta, qv
     ub += 0.5f * r * (LD(a.mb[0], id) + LD(a.mb[0], row + j * nx + ip));                // u
     ub += 0.5f * r * (LD(a.mb[1], id) + LD(a.mb[1], row + wrapx(j + 1, ny) * nx + i));  // v (corner)
     ub += 0.5f * r * ((k >= 1 ? LD(a.mb[2], id) : 0.f) + (k + 1 < nz ? LD(a.mb[2], id + plane) : 0.f));  // w
@@ -766,7 +751,7 @@ __global__ void __launch_bounds__(AB) k_adv_gather_vjp(Dims d, Phys ph, Cols c, 
     if (k >= nz) return;
     const float r = c.rho[k];
     const int row = k * plane;
-    float vb = r * (LD(a.mb[3], id) + LD(a.P[0][0], id));
+    float vb = r * (LD(a.mb[3], id) + LD(a.mb[4], id));
     vb += 0.5f * r * (LD(a.mb[0], id) + LD(a.mb[0], row + j * nx + ip));
     vb += 0.5f * r * (LD(a.mb[1], id) + LD(a.mb[1], row + jp * nx + i));
     vb += 0.5f * r * ((k >= 1 ? LD(a.mb[2], id) : 0.f) + (k + 1 < nz ? LD(a.mb[2], id + plane) : 0.f));
@@ -776,7 +761,7 @@ __global__ void __launch_bounds__(AB) k_adv_gather_vjp(Dims d, Phys ph, Cols c, 
     float wb = 0.f;
     if (k >= 1 && k < nz) {
       const float rf = c.rho_face[k];
-      wb += rf * (LD(a.mb[3], id) + LD(a.P[0][0], id));
+      wb += rf * (LD(a.mb[3], id) + LD(a.mb[4], id));
       wb += 0.5f * rf * (LD(a.mb[0], id) + LD(a.mb[0], row + j * nx + ip));
       wb += 0.5f * rf * (LD(a.mb[1], id) + LD(a.mb[1], row + jp * nx + i));
     }
@@ -1141,16 +1126,25 @@ static cudaError_t launch_march(const Dims& d, const Phys& ph, const Cols& c, co
   return cudaGetLastError();
 }
 
+// whole rows, as many as ROW_T threads take, or segments of long ones
+static cudaError_t launch_rows(const Dims& d, const Phys& ph, const Cols& c, const AdvVjpArgs& a, cudaStream_t st) {
+  const int rows = d.nx <= ROW_T ? ROW_T / d.nx : 0;
+  const long long all = (long long)d.ny * (d.nz + 1);
+  const dim3 g((unsigned)(rows ? (all + rows - 1) / rows : all), rows ? 1 : (d.nx + ROW_T - 6) / (ROW_T - 5));
+  const int threads = rows ? (rows * d.nx + 31) / 32 * 32 : ROW_T;
+  k_adv_row_vjp<<<g, threads, 0, st>>>(d, ph, c, a, rows);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_adv_vjp(const Dims& d, const Phys& ph, const Cols& c, const AdvVjpArgs& a, cudaStream_t st) {
   const unsigned g = (unsigned)((d.faces() + AB - 1) / AB);
-  k_adv_face_vjp<0><<<g, AB, 0, st>>>(d, ph, c, a);
-  k_adv_gather_vjp<0><<<g, AB, 0, st>>>(d, ph, c, a);
-  cudaError_t e = launch_march<1>(d, ph, c, a, st);
+  cudaError_t e = launch_rows(d, ph, c, a, st);
   if (e != cudaSuccess) return e;
-  k_adv_gather_vjp<1><<<g, AB, 0, st>>>(d, ph, c, a);
-  e = launch_march<2>(d, ph, c, a, st);
-  if (e != cudaSuccess) return e;
-  k_adv_gather_vjp<2><<<g, AB, 0, st>>>(d, ph, c, a);
+  k_adv_mass_vjp<0><<<g, AB, 0, st>>>(d, ph, c, a);
+  if ((e = launch_march<1>(d, ph, c, a, st)) != cudaSuccess) return e;
+  k_adv_mass_vjp<1><<<g, AB, 0, st>>>(d, ph, c, a);
+  if ((e = launch_march<2>(d, ph, c, a, st)) != cudaSuccess) return e;
+  k_adv_mass_vjp<2><<<g, AB, 0, st>>>(d, ph, c, a);
   return cudaGetLastError();
 }
 

@@ -35,8 +35,7 @@ struct AdvVjpArgs {
   State xs;              // stage input (winds for the mass fluxes)
   const float* phi[5];   // advected fields u, v, w, T, q
   const float* cb[5];
-  float* P[5][6];        // per-flux stencil adjoints, slot q = point p-3+q of the flux between p-1, p
-  float* mb[4];          // mass-flux adjoints: u, v, w fluxes and theta+qv fluxes
+  float* mb[5];          // mass-flux adjoints of the fields' fluxes
   State xsb;             // accumulated
 };
 

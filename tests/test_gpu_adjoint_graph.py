@@ -55,8 +55,8 @@ def test_repeated_reverse_passes_agree(built_lib, dims):
 
 
 @pytest.mark.parametrize("nx,ny,nz,copies,axis", [(15, 13, 9, 4, 2), (30, 13, 9, 2, 2), (44, 13, 9, 2, 2),
-                                                  (16, 4, 6, 9, 1), (12, 5, 33, 10, 1)],
-                         ids=["odd rows", "even rows", "rows of four", "four rows", "five rows, high"])
+                                                  (150, 5, 6, 2, 2), (16, 4, 6, 9, 1), (12, 5, 33, 10, 1)],
+                         ids=["odd rows", "even rows", "rows of four", "long rows", "four rows", "five rows, high"])
 def test_reverse_pass_on_periodic_copies(built_lib, nx, ny, nz, copies, axis):
     """Periodic copies side by side are the same flow, so a grid and one of `copies` times as many points in x
     or y give the same step and the same adjoint.  The kernels take one, two or four cells a thread by the

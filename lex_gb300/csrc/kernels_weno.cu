@@ -101,8 +101,7 @@ __device__ __forceinline__ float2 vflux6x2(float m, float2 sm3, float2 sm2, floa
 // ================================================================================================
 // theta and qv, vertical march
 //
-// A block owns 32 x 8 columns (one thread each) and marches up a chunk of levels (as many chunks
-// as make one wave of resident blocks: zm_chunk).  For the x and
+// A block owns 32 x 8 columns (one thread each) and marches up a chunk of levels (zm_chunk).  For the x and
 // y faces of a level it stages that level's plane of theta and qv with a 3-cell halo (40 x 14
 // values, x widened to 4-aligned 16-byte pieces) by cp.async into a two-slot ring, the next level's
 // plane in flight while the current one is used; the vertical stencil of a thread's own column
@@ -126,13 +125,17 @@ constexpr int kScalarsZmBlocks = 3;   // resident blocks per SM the theta/qv mar
 int g_zm_slots = 304, g_zs_slots = 608;
 
 // levels per block of a vertical march: as many level chunks as make one wave of resident blocks, down
-// to single levels.  A chunk costs about one level more than it owns, but a small grid is bound by the
-// serial march: theta/qv + u,v,w at 16x16x12 take 53 us in chunks of 8 levels and 14.5 us in chunks of
-// 1, 32^3 39 and 14.5, 64^3 41 and 31 (chunks of 3); from 128x128x64 on the chunks are longer than 8.
+// to single levels, and at most nine levels.  A chunk costs about one level more than it owns, but a small
+// grid is bound by the serial march: theta/qv + u,v,w at 16x16x12 take 53 us in chunks of 8 levels and
+// 14.5 us in chunks of 1, 32^3 39 and 14.5, 64^3 41 and 31 (chunks of 3).  And where one wave leaves SMs
+// with a block less than others, for the whole march, short chunks even that out; a step with one wave,
+// 6, 9 and 16 levels: 240x240x120 (240 tiles on 456 places) 4.74, 4.21, 4.16, 4.16 ms, 320x200x60 2.53,
+// 2.32, 2.29, 2.32, 256x256x64 3.04, 2.82, 2.79, 2.83, 192x192x96 2.16, 2.17, 2.14, 2.16, 128x128x64
+// 0.68, 0.69, 0.67, 0.68.
 inline int zm_chunk(const Dims& d, int slots) {
   const int tiles = ((d.nx + 31) / 32) * ((d.ny + 7) / 8);
   const int nch = max(1, min(slots / tiles, d.nz));
-  return (d.nz + nch - 1) / nch;
+  return min((d.nz + nch - 1) / nch, 9);
 }
 
 __device__ __forceinline__ void cp_async16(unsigned sa, const void* gmem) {

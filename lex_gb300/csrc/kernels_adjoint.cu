@@ -1,21 +1,20 @@
 // kernels_adjoint.cu - vector-Jacobian products (reverse mode) of the big-step operators.
 //
-// Every kernel is a gather: a thread owns one output adjoint value and sums the contributions
-// of the forward outputs that depend on it, so there are no atomics and the results do not
-// depend on scheduling.  The forward operators and their reference counterparts:
+// A thread owns the adjoint values it writes and sums the contributions of the forward outputs that
+// depend on them, so there are no atomics and the results do not depend on scheduling.  The forward
+// operators and their reference counterparts:
 //
 //   acoustic sub-step        one_step_integration.py:519-556 (k_acoustic_vec)
-//   WENO flux divergence     advection.py:9-149, fluxes :305-1281 (k_weno_scalars/momentum)
+//   WENO flux divergence     advection.py:9-149, fluxes :305-1281 (k_weno_scalars_zm/momentum_zm)
 //   mass divergence          advection.py:200-226 (k_div_trho)
 //   theta_rho, buoyancy      one_step_integration.py:269, pressure_equations.py:162-172
 //   Coriolis                 pressure_gradient_coriolis.py:80-113
 //
-// WENO adjoint: for each direction a face kernel evaluates, for every flux of the five advected
-// fields (theta, qv, u, v, w), the flux adjoint Fbar = (cbar(right) - cbar(left)) / dx, the
-// reconstruction W and its derivatives with respect to its stencil, and stores
-// Fbar * m * dW/ds as six slots (the cells p-3 .. p+2 of the flux between p-1 and p) plus the
-// mass-flux adjoint Fbar * W.  A gather kernel then adds, for every point, the six slots that
-// name it and the mass-flux adjoints of the fluxes whose mass flux it enters.
+// WENO adjoint: for each direction and every flux of the five advected fields (u, v, w, theta, qv), the
+// flux adjoint Fbar = (cbar(right) - cbar(left)) / dx, the reconstruction W and its derivatives with
+// respect to its stencil.  Fbar * m * dW/ds goes, as six slots, to the points p-3 .. p+2 of the flux between
+// p-1 and p (k_adv_row_vjp, k_adv_march_vjp); the mass-flux adjoints Fbar * W go to the winds whose mass
+// flux they are in a second kernel (k_adv_mass_vjp).
 #include "lexgb_adjoint.cuh"
 #include "smag_ops.cuh"
 

@@ -46,7 +46,10 @@ __device__ __forceinline__ float adv_pi(const Dims& d, const Phys& ph, const Col
 }
 
 // Each thread owns V (4, 2 or 1) consecutive x points of one (j, k) row and moves every field with
-// V-wide loads/stores (needs nx % V == 0).
+// V-wide loads/stores (needs nx % V == 0).  For V = 2 and 1 the products that are added without a rounding
+// of their own are written out (div, ax, ay, az, dpdt): left to the compiler, they were others than those of
+// one cell a thread, which served these rows before, and pi' differed from it in the last bit of a fifth of the
+// cells.  That much moves the sign of a mass flux somewhere, and an adjoint jumps there.
 template <int V>
 struct VecT;
 template <>
@@ -191,15 +194,24 @@ __global__ void __launch_bounds__(V == 4 ? 64 : 128, V == 4 ? 8 : 6) k_acoustic_
     const float vn = VN[l] + (pgf(TN[l], t0, PN[l], p0, ph.rdy) + RVN[l]) * dtau;
     const float wb = has_b ? W[l] + (pgf(t0, TB[l], p0, PB[l], ph.rdz) + RW[l]) * dtau : 0.f;
     const float wt = has_t ? WT[l] + (pgf(TT[l], t0, PT[l], p0, ph.rdz) + RWT[l]) * dtau : 0.f;
-    const float div = (un[l + 1] - un[l]) * ph.rdx + (vn - vs) * ph.rdy + (wt - wb) * ph.rdz;
+    const float div =
+        V == 4 ? (un[l + 1] - un[l]) * ph.rdx + (vn - vs) * ph.rdy + (wt - wb) * ph.rdz
+               : __fmaf_rn(wt - wb, ph.rdz, __fmaf_rn(un[l + 1] - un[l], ph.rdx, __fmul_rn(vn - vs, ph.rdy)));
     const float s0 = sc[l + 1];
     const float gxw = (s0 - sc[l]) * ph.rdx, gxe = (sc[l + 2] - s0) * ph.rdx;
     const float gys = (s0 - SS[l]) * ph.rdy, gyn = (SN[l] - s0) * ph.rdy;
     const float wzb = has_b ? wb * (dzb + (s0 - SB[l]) * ph.rdz) : 0.f;
     const float wzt = has_t ? wt * (dzt + (ST[l] - s0) * ph.rdz) : 0.f;
-    const float ap = -(0.5f * (un[l + 1] * gxe + un[l] * gxw) + 0.5f * (vn * gyn + vs * gys) +
-                       (0.5f * wzb * rfb + 0.5f * wzt * rft) * rhoi);
-    const float dpdt = -kRdCv * ((pi0 + s0) * div) + ap;
+    float dpdt;
+    if (V == 4) {
+      const float ap = -(0.5f * (un[l + 1] * gxe + un[l] * gxw) + 0.5f * (vn * gyn + vs * gys) +
+                         (0.5f * wzb * rfb + 0.5f * wzt * rft) * rhoi);
+      dpdt = -kRdCv * ((pi0 + s0) * div) + ap;
+    } else {
+      const float ax = __fmaf_rn(un[l], gxw, __fmul_rn(un[l + 1], gxe)), ay = __fmaf_rn(vs, gys, __fmul_rn(vn, gyn));
+      const float az = __fmaf_rn(0.5f * wzb, rfb, __fmul_rn(0.5f * wzt, rft));
+      dpdt = __fmaf_rn(-kRdCv, (pi0 + s0) * div, -__fmaf_rn(az, rhoi, 0.5f * ax + 0.5f * ay));
+    }
     outp[l] = p0 + (kDivDamp * dpdt) * dtau;
     outv[l] = vs;
     outw[l] = wb;

@@ -30,6 +30,7 @@ __device__ __forceinline__ int pmod(int i, int n) {
 // face value through column face H (between entries H-1 and H of an n-entry column), given
 // s(H-3..H+2); entries outside 0..n-1 are never used; zero on the end faces.  Near-boundary
 // rules of vertical_flux_scalar2 and friends (advection.py:327-406).
+template <bool B2 = false>
 __device__ __forceinline__ float vflux6(float m, float sm3, float sm2, float sm1, float s0, float sp1, float sp2, int H,
                                         int n, float eps) {
   if (H <= 0 || H >= n) return 0.f;
@@ -43,7 +44,7 @@ __device__ __forceinline__ float vflux6(float m, float sm3, float sm2, float sm1
     else if (H == 2 || H == n - 1)
       r = weno3(sm2, sm1, s0, eps);
     else  // H == n-2
-      r = weno5(sm3, sm2, sm1, s0, sp1, eps);
+      r = weno5<B2>(sm3, sm2, sm1, s0, sp1, eps);
   } else {
     if (H == n - 1)
       r = 0.5f * (s0 + sm1);
@@ -110,9 +111,13 @@ __device__ __forceinline__ float2 vflux6x2(float m, float2 sm3, float2 sm2, floa
 // (the mass-flux winds and the stencil's next column value are loaded one level ahead)
 // warp 1 the 32 north-edge y faces.  The bottom face of level k+1 is the top face of level k, so a
 // level's tendency is completed in the next iteration.  Rows that do not start on 16-byte
-// boundaries (nx % 4 != 0) are staged in 4-byte pieces (Stager): 102x75x59 21.7 us (theta, qv) and
-// 31.8 us (u, v, w); one 32 x 4 x 4 box with a 3-D halo per block took 27.2 (with a kernel of its own
-// for the divergence) and 37.5.
+// boundaries (nx % 4 != 0) are staged in 4-byte pieces (Stager): 102x75x59 22.5 us (theta, qv) and
+// 36.9 us (u, v, w); one 32 x 4 x 4 box with a 3-D halo per block took 27.2 (with a kernel of its own
+// for the divergence) and 37.5.  On such rows (V16 false) the marches keep the boxes' arithmetic, bit
+// for bit: divisions by rho0, u, v and w reconstructed one by one, products and sums contracted as diff,
+// mean, sum2 and sum3 say.  In the other rows' arithmetic (reciprocals, packed reconstructions) u, v and w
+// took 31.8 us, and the states differed in their last bits: that much moves the sign of a mass flux
+// somewhere, where an adjoint jumps (up to 3e-3 of its rms at single points).
 // ================================================================================================
 constexpr int ZX = 32, ZY = 8, ZHX = 4, ZHY = 3;
 constexpr int ZPX = ZX + 2 * ZHX, ZPY = ZY + 2 * ZHY;   // staged plane 40 x 14
@@ -199,6 +204,17 @@ struct ZLevel {
   float2 top;   // the column value three levels up, for the register stencil
 };
 
+// Products and sums of the marches on rows of other lengths than multiples of 4, each rounded as written.
+// r a - s b, 0.5 (r a + s b) and a da + b db + c dc:
+__device__ __forceinline__ float diff(float r, float a, float s, float b) { return __fmaf_rn(r, a, -__fmul_rn(s, b)); }
+__device__ __forceinline__ float mean(float r, float a, float s, float b) {
+  return 0.5f * __fmaf_rn(r, a, __fmul_rn(s, b));
+}
+__device__ __forceinline__ float sum2(float a, float da, float b, float db) { return __fmaf_rn(a, da, __fmul_rn(b, db)); }
+__device__ __forceinline__ float sum3(float a, float da, float b, float db, float c, float dc) {
+  return __fmaf_rn(c, dc, sum2(a, da, b, db));
+}
+
 // FUSED: also form div(rho0 u) and theta_rho of the state (a.div_out, a.trho_out) instead of reading a.div
 template <bool FUSED, bool V16>
 __global__ void __launch_bounds__(ZNT, kScalarsZmBlocks) k_weno_scalars_zm(Dims d, Phys ph, Cols c, State s,
@@ -270,10 +286,11 @@ __global__ void __launch_bounds__(ZNT, kScalarsZmBlocks) k_weno_scalars_zm(Dims 
     if (k > kb && col_own) {  // level k-1 complete
       const int km = k - 1;
       const size_t id = (size_t)km * plane + cidx;
-      const float ri = c.rho_inv[km];
+      const float ri = V16 ? c.rho_inv[km] : c.rho[km];
       const float2 cv = fma2(sub2(zf, zprev), f2(-ph.rdz), inner);
-      const float advT = (cv.x + own.x * dv) * ri;   // 1/rho0 as a correctly rounded column value
-      const float advQ = (cv.y + own.y * dv) * ri;
+      // 1/rho0 as a correctly rounded column value, or a division
+      const float advT = V16 ? (cv.x + own.x * dv) * ri : (cv.x + own.x * dv) / ri;
+      const float advQ = V16 ? (cv.y + own.y * dv) * ri : (cv.y + own.y * dv) / ri;
       float Tn = T0 + advT * a.dts, Qn = Q0 + advQ * a.dts, rT = advT, rQ = advQ;
       if (a.sgsT) {
         Tn = Tn + sT * a.dts;
@@ -314,11 +331,12 @@ __global__ void __launch_bounds__(ZNT, kScalarsZmBlocks) k_weno_scalars_zm(Dims 
     own = v2(ly, lx);
     float dvz = 0.f;
     if (fused) {
-      sMx[ty][tx] = mx;
-      sMy[ty][tx] = my;
-      if (ty == 0 && tx < ZY) sMx[tx][ZX] = mxe;
-      if (ty == 1) sMy[ZY][tx] = mye;
-      dvz = (c.rho_face0[k + 1] * nxt.w - c.rho_face0[k] * cur.w) * ph.rdz;
+      sMx[ty][tx] = V16 ? mx : cur.u;
+      sMy[ty][tx] = V16 ? my : cur.v;
+      if (ty == 0 && tx < ZY) sMx[tx][ZX] = V16 ? mxe : cur.ue;
+      if (ty == 1) sMy[ZY][tx] = V16 ? mye : cur.ve;
+      dvz = V16 ? (c.rho_face0[k + 1] * nxt.w - c.rho_face0[k] * cur.w) * ph.rdz
+                : diff(c.rho_face0[k + 1], nxt.w, c.rho_face0[k], cur.w);
     }
     xF[ty][tx] = weno_flux_x2(mx, v2(ly, lx - 3), v2(ly, lx - 2), v2(ly, lx - 1), v2(ly, lx), v2(ly, lx + 1),
                               v2(ly, lx + 2), eps);
@@ -337,9 +355,14 @@ __global__ void __launch_bounds__(ZNT, kScalarsZmBlocks) k_weno_scalars_zm(Dims 
     __syncthreads();
     inner = fma2(sub2(yF[ty + 1][tx], yF[ty][tx]), f2(-ph.rdy), mul2(sub2(xF[ty][tx + 1], xF[ty][tx]), f2(-ph.rdx)));
     if (fused && col_own) {  // get_divergence (advection.py:200-226) and theta_rho, as k_div_trho forms them
-      const float dvx = (sMx[ty][tx + 1] - sMx[ty][tx]) * ph.rdx;
-      const float dvy = (sMy[ty + 1][tx] - sMy[ty][tx]) * ph.rdy;
-      dv = dvx + dvy + dvz;
+      if (V16) {
+        const float dvx = (sMx[ty][tx + 1] - sMx[ty][tx]) * ph.rdx;
+        const float dvy = (sMy[ty + 1][tx] - sMy[ty][tx]) * ph.rdy;
+        dv = dvx + dvy + dvz;
+      } else {
+        dv = sum3(diff(r, sMx[ty][tx + 1], r, sMx[ty][tx]), ph.rdx, diff(r, sMy[ty + 1][tx], r, sMy[ty][tx]), ph.rdy,
+                  dvz, ph.rdz);
+      }
       const size_t id = (size_t)k * plane + cidx;
       a.div_out[id] = dv;
       a.trho_out[id] = theta_rho(own.x, own.y, ph.theta_ref);
@@ -386,8 +409,12 @@ __device__ __forceinline__ float2 sel2m(bool p, bool q, float2 a, float2 b) {
 
 // (m.x * upwind WENO5 of stencil .x, m.y * upwind WENO5 of stencil .y): two faces with mass fluxes of
 // their own
+template <bool PACKED>
 __device__ __forceinline__ float2 weno_flux_2m(float2 m, float2 sm3, float2 sm2, float2 sm1, float2 s0, float2 sp1,
                                                float2 sp2, float2 eps) {
+  if (!PACKED)
+    return make_float2(weno_flux(m.x, sm3.x, sm2.x, sm1.x, s0.x, sp1.x, sp2.x, eps.x),
+                       weno_flux(m.y, sm3.y, sm2.y, sm1.y, s0.y, sp1.y, sp2.y, eps.y));
   const bool p = m.x >= 0.f, q = m.y >= 0.f;
   return mul2(m, weno5x2(sel2m(p, q, sm3, sp2), sel2m(p, q, sm2, sp1), sel2m(p, q, sm1, s0), sel2m(p, q, s0, sm1),
                          sel2m(p, q, sp1, sm2), eps));
@@ -395,12 +422,13 @@ __device__ __forceinline__ float2 weno_flux_2m(float2 m, float2 sm3, float2 sm2,
 
 // vflux6 for two columns at the same face H: packed away from the ends, where each column's
 // direction picks its own near-boundary rule
+template <bool PACKED>
 __device__ __forceinline__ float2 vflux6_2m(float2 m, float2 sm3, float2 sm2, float2 sm1, float2 s0, float2 sp1,
                                             float2 sp2, int H, int n, float eps) {
   if (H <= 0 || H >= n) return f2(0.f);
-  if (H >= 3 && H <= n - 3) return weno_flux_2m(m, sm3, sm2, sm1, s0, sp1, sp2, f2(eps));
-  return make_float2(vflux6(m.x, sm3.x, sm2.x, sm1.x, s0.x, sp1.x, sp2.x, H, n, eps),
-                     vflux6(m.y, sm3.y, sm2.y, sm1.y, s0.y, sp1.y, sp2.y, H, n, eps));
+  if (PACKED && H >= 3 && H <= n - 3) return weno_flux_2m<true>(m, sm3, sm2, sm1, s0, sp1, sp2, f2(eps));
+  return make_float2(vflux6<!PACKED>(m.x, sm3.x, sm2.x, sm1.x, s0.x, sp1.x, sp2.x, H, n, eps),
+                     vflux6<!PACKED>(m.y, sm3.y, sm2.y, sm1.y, s0.y, sp1.y, sp2.y, H, n, eps));
 }
 
 
@@ -501,10 +529,11 @@ __global__ void __launch_bounds__(ZNT, 3) k_weno_momentum_zm(Dims d, Phys ph, Co
     float2 zUV = f2(0.f);
     if (k >= 1 && k < nz) {
       const float rf = c.rho_face[k];
-      const float2 m = make_float2(0.5f * (rf * PW[ly][lx - 1] + rf * PW[ly][lx]),
-                                   0.5f * (rf * PW[ly - 1][lx] + rf * PW[ly][lx]));
-      zUV = vflux6_2m(m, make_float2(su[0], sv[0]), make_float2(su[1], sv[1]), make_float2(su[2], sv[2]),
-                      make_float2(su[3], sv[3]), make_float2(su[4], sv[4]), make_float2(su[5], sv[5]), k, nz, eps);
+      const float2 m = V16 ? make_float2(0.5f * (rf * PW[ly][lx - 1] + rf * PW[ly][lx]),
+                                         0.5f * (rf * PW[ly - 1][lx] + rf * PW[ly][lx]))
+                           : make_float2(mean(rf, PW[ly][lx - 1], rf, PW[ly][lx]), mean(rf, PW[ly - 1][lx], rf, PW[ly][lx]));
+      zUV = vflux6_2m<V16>(m, make_float2(su[0], sv[0]), make_float2(su[1], sv[1]), make_float2(su[2], sv[2]),
+                           make_float2(su[3], sv[3]), make_float2(su[4], sv[4]), make_float2(su[5], sv[5]), k, nz, eps);
     }
     const float zW = (k >= 1) ? vflux6(0.5f * (sw[2] + sw[3]) * c.rho[k - 1], sw[0], sw[1], sw[2], sw[3], sw[4],
                                        sw[5], k, nz + 1, eps)
@@ -512,13 +541,24 @@ __global__ void __launch_bounds__(ZNT, 3) k_weno_momentum_zm(Dims d, Phys ph, Co
     if (k > kb && col_own) {  // level k-1 complete
       const int kk = k - 1;
       const size_t id = (size_t)kk * plane + cidx;
-      const float ri = c.rho_inv[kk];   // 1/rho0, 1/rho0 on the face: correctly rounded column values
-      const float2 cuv = fma2(sub2(zUV, zpUV), f2(-ph.rdz), inUV);
-      float Ru = (cuv.x + su[2] * (0.5f * (dxC + dcC))) * ri;
-      float Rv = (cuv.y + sv[2] * (0.5f * (dyC + dcC))) * ri;
-      if (ph.cor_opt) {
-        Ru = Ru + corU;
-        Rv = Rv - corV;
+      float Ru, Rv;
+      if (V16) {
+        const float ri = c.rho_inv[kk];   // 1/rho0, 1/rho0 on the face: correctly rounded column values
+        const float2 cuv = fma2(sub2(zUV, zpUV), f2(-ph.rdz), inUV);
+        Ru = (cuv.x + su[2] * (0.5f * (dxC + dcC))) * ri;
+        Rv = (cuv.y + sv[2] * (0.5f * (dyC + dcC))) * ri;
+        if (ph.cor_opt) {
+          Ru = Ru + corU;
+          Rv = Rv - corV;
+        }
+      } else {
+        const float r1 = c.rho[kk];
+        Ru = (su[2] * (0.5f * (dxC + dcC)) - __fmaf_rn(__fsub_rn(zUV.x, zpUV.x), ph.rdz, inUV.x)) / r1;
+        Rv = (sv[2] * (0.5f * (dyC + dcC)) - __fmaf_rn(__fsub_rn(zUV.y, zpUV.y), ph.rdz, inUV.y)) / r1;
+        if (ph.cor_opt) {
+          Ru = __fmaf_rn(ph.f_cor * 0.25f, corU, Ru);
+          Rv = __fmaf_rn(-ph.f_cor, corV, Rv);
+        }
       }
       if (a.sgs_u) {
         Ru = Ru + sgU;
@@ -528,8 +568,12 @@ __global__ void __launch_bounds__(ZNT, 3) k_weno_momentum_zm(Dims d, Phys ph, Co
       a.Rv[id] = Rv;
       float adv = 0.f;   // w on face kk
       if (kk >= 1) {
-        const float cw = fmaf(zW - zpW, -ph.rdz, inW);
-        adv = (cw + sw[2] * (0.5f * (dzC + dcC))) * c.rho_w_inv[kk];
+        if (V16) {
+          const float cw = fmaf(zW - zpW, -ph.rdz, inW);
+          adv = (cw + sw[2] * (0.5f * (dzC + dcC))) * c.rho_w_inv[kk];
+        } else {
+          adv = (sw[2] * (0.5f * (dzC + dcC)) - __fmaf_rn(zW - zpW, ph.rdz, inW)) / (0.5f * (c.rho[kk - 1] + c.rho[kk]));
+        }
       }
       float Rw = adv;
       if (a.wmode != 1) {
@@ -551,29 +595,32 @@ __global__ void __launch_bounds__(ZNT, 3) k_weno_momentum_zm(Dims d, Phys ph, Co
     auto xs = [&](const float(&P)[ZPY][ZPX], int ry, int rx, int o) { return P[ry][rx + o]; };
     {
       const float2 mu = make_float2(0.5f * (PU[ly][lx - 1] + PU[ly][lx]) * r,          // cell between u's
-                                    0.5f * (r * PV[ly][lx - 1] + r * PV[ly][lx]));     // corner
-      const float2 fu = weno_flux_2m(mu, make_float2(PU[ly][lx - 3], PU[ly - 3][lx]),
-                                     make_float2(PU[ly][lx - 2], PU[ly - 2][lx]),
-                                     make_float2(PU[ly][lx - 1], PU[ly - 1][lx]), make_float2(PU[ly][lx], PU[ly][lx]),
-                                     make_float2(PU[ly][lx + 1], PU[ly + 1][lx]),
-                                     make_float2(PU[ly][lx + 2], PU[ly + 2][lx]), f2(eps));
-      const float2 mv = make_float2(0.5f * (r * PU[ly - 1][lx] + r * PU[ly][lx]),      // corner
+                                    V16 ? 0.5f * (r * PV[ly][lx - 1] + r * PV[ly][lx])     // corner
+                                        : mean(r, PV[ly][lx - 1], r, PV[ly][lx]));
+      const float2 fu = weno_flux_2m<V16>(mu, make_float2(PU[ly][lx - 3], PU[ly - 3][lx]),
+                                          make_float2(PU[ly][lx - 2], PU[ly - 2][lx]),
+                                          make_float2(PU[ly][lx - 1], PU[ly - 1][lx]), make_float2(PU[ly][lx], PU[ly][lx]),
+                                          make_float2(PU[ly][lx + 1], PU[ly + 1][lx]),
+                                          make_float2(PU[ly][lx + 2], PU[ly + 2][lx]), f2(eps));
+      const float2 mv = make_float2(V16 ? 0.5f * (r * PU[ly - 1][lx] + r * PU[ly][lx])      // corner
+                                        : mean(r, PU[ly - 1][lx], r, PU[ly][lx]),
                                     0.5f * (PV[ly - 1][lx] + PV[ly][lx]) * r);         // cell between v's
-      const float2 fv = weno_flux_2m(mv, make_float2(PV[ly][lx - 3], PV[ly - 3][lx]),
-                                     make_float2(PV[ly][lx - 2], PV[ly - 2][lx]),
-                                     make_float2(PV[ly][lx - 1], PV[ly - 1][lx]), make_float2(PV[ly][lx], PV[ly][lx]),
-                                     make_float2(PV[ly][lx + 1], PV[ly + 1][lx]),
-                                     make_float2(PV[ly][lx + 2], PV[ly + 2][lx]), f2(eps));
+      const float2 fv = weno_flux_2m<V16>(mv, make_float2(PV[ly][lx - 3], PV[ly - 3][lx]),
+                                          make_float2(PV[ly][lx - 2], PV[ly - 2][lx]),
+                                          make_float2(PV[ly][lx - 1], PV[ly - 1][lx]), make_float2(PV[ly][lx], PV[ly][lx]),
+                                          make_float2(PV[ly][lx + 1], PV[ly + 1][lx]),
+                                          make_float2(PV[ly][lx + 2], PV[ly + 2][lx]), f2(eps));
       xUV[ty][tx] = make_float2(fu.x, fv.x);
       yUV[ty][tx] = make_float2(fu.y, fv.y);
     }
     if (k >= 1 && k < nz) {  // w's lateral faces on interior face levels
-      const float2 mw = make_float2(0.5f * (rm * su[2] + r * su[3]), 0.5f * (rm * sv[2] + r * sv[3]));
-      const float2 fw = weno_flux_2m(mw, make_float2(PW[ly][lx - 3], PW[ly - 3][lx]),
-                                     make_float2(PW[ly][lx - 2], PW[ly - 2][lx]),
-                                     make_float2(PW[ly][lx - 1], PW[ly - 1][lx]), make_float2(PW[ly][lx], PW[ly][lx]),
-                                     make_float2(PW[ly][lx + 1], PW[ly + 1][lx]),
-                                     make_float2(PW[ly][lx + 2], PW[ly + 2][lx]), f2(eps));
+      const float2 mw = V16 ? make_float2(0.5f * (rm * su[2] + r * su[3]), 0.5f * (rm * sv[2] + r * sv[3]))
+                            : make_float2(mean(rm, su[2], r, su[3]), mean(rm, sv[2], r, sv[3]));
+      const float2 fw = weno_flux_2m<V16>(mw, make_float2(PW[ly][lx - 3], PW[ly - 3][lx]),
+                                          make_float2(PW[ly][lx - 2], PW[ly - 2][lx]),
+                                          make_float2(PW[ly][lx - 1], PW[ly - 1][lx]), make_float2(PW[ly][lx], PW[ly][lx]),
+                                          make_float2(PW[ly][lx + 1], PW[ly + 1][lx]),
+                                          make_float2(PW[ly][lx + 2], PW[ly + 2][lx]), f2(eps));
       xW[ty][tx] = fw.x;
       yW[ty][tx] = fw.y;
     } else {
@@ -582,34 +629,43 @@ __global__ void __launch_bounds__(ZNT, 3) k_weno_momentum_zm(Dims d, Phys ph, Co
     }
     float corUN = 0.f, corVN = 0.f;
     if (ph.cor_opt) {  // f v at u points, f u at v points (4-point averages)
-      corUN = ph.f_cor * 0.25f * (PV[ly][lx - 1] + PV[ly + 1][lx - 1] + PV[ly][lx] + PV[ly + 1][lx]);
-      const float fu = 0.25f * (PU[ly - 1][lx] + PU[ly][lx] + PU[ly - 1][lx + 1] + PU[ly][lx + 1]);
-      corVN = ph.cor_opt == 2 ? ph.f_cor * (fu - 1.0f) : ph.f_cor * fu;
+      if (V16) {
+        corUN = ph.f_cor * 0.25f * (PV[ly][lx - 1] + PV[ly + 1][lx - 1] + PV[ly][lx] + PV[ly + 1][lx]);
+        const float fu = 0.25f * (PU[ly - 1][lx] + PU[ly][lx] + PU[ly - 1][lx + 1] + PU[ly][lx + 1]);
+        corVN = ph.cor_opt == 2 ? ph.f_cor * (fu - 1.0f) : ph.f_cor * fu;
+      } else {   // without the factors, which come with the sum they are added to
+        corUN = PV[ly][lx - 1] + PV[ly + 1][lx - 1] + PV[ly][lx] + PV[ly + 1][lx];
+        corVN = 0.25f * (PU[ly - 1][lx] + PU[ly][lx] + PU[ly - 1][lx + 1] + PU[ly][lx + 1]);
+        if (ph.cor_opt == 2) corVN = corVN - 1.0f;
+      }
     }
     if (ty == 0 && tx < ZY) {  // east x faces of u and v, row tx
       const int ry = tx + ZHY, rx = ZX + ZHX;
       const float2 m = make_float2(0.5f * (PU[ry][rx - 1] + PU[ry][rx]) * r,
-                                   0.5f * (r * PU[ry - 1][rx] + r * PU[ry][rx]));
-      xUV[tx][ZX] = weno_flux_2m(m, make_float2(xs(PU, ry, rx, -3), xs(PV, ry, rx, -3)),
-                                 make_float2(xs(PU, ry, rx, -2), xs(PV, ry, rx, -2)),
-                                 make_float2(xs(PU, ry, rx, -1), xs(PV, ry, rx, -1)),
-                                 make_float2(xs(PU, ry, rx, 0), xs(PV, ry, rx, 0)),
-                                 make_float2(xs(PU, ry, rx, 1), xs(PV, ry, rx, 1)),
-                                 make_float2(xs(PU, ry, rx, 2), xs(PV, ry, rx, 2)), f2(eps));
+                                   V16 ? 0.5f * (r * PU[ry - 1][rx] + r * PU[ry][rx])
+                                       : mean(r, PU[ry - 1][rx], r, PU[ry][rx]));
+      xUV[tx][ZX] = weno_flux_2m<V16>(m, make_float2(xs(PU, ry, rx, -3), xs(PV, ry, rx, -3)),
+                                      make_float2(xs(PU, ry, rx, -2), xs(PV, ry, rx, -2)),
+                                      make_float2(xs(PU, ry, rx, -1), xs(PV, ry, rx, -1)),
+                                      make_float2(xs(PU, ry, rx, 0), xs(PV, ry, rx, 0)),
+                                      make_float2(xs(PU, ry, rx, 1), xs(PV, ry, rx, 1)),
+                                      make_float2(xs(PU, ry, rx, 2), xs(PV, ry, rx, 2)), f2(eps));
     } else if (ty == 1) {  // north y faces of u and v, column tx
       const int ry = ZY + ZHY, rx = tx + ZHX;
-      const float2 m = make_float2(0.5f * (r * PV[ry][rx - 1] + r * PV[ry][rx]),
+      const float2 m = make_float2(V16 ? 0.5f * (r * PV[ry][rx - 1] + r * PV[ry][rx])
+                                       : mean(r, PV[ry][rx - 1], r, PV[ry][rx]),
                                    0.5f * (PV[ry - 1][rx] + PV[ry][rx]) * r);
-      yUV[ZY][tx] = weno_flux_2m(m, make_float2(PU[ry - 3][rx], PV[ry - 3][rx]),
-                                 make_float2(PU[ry - 2][rx], PV[ry - 2][rx]),
-                                 make_float2(PU[ry - 1][rx], PV[ry - 1][rx]), make_float2(PU[ry][rx], PV[ry][rx]),
-                                 make_float2(PU[ry + 1][rx], PV[ry + 1][rx]),
-                                 make_float2(PU[ry + 2][rx], PV[ry + 2][rx]), f2(eps));
+      yUV[ZY][tx] = weno_flux_2m<V16>(m, make_float2(PU[ry - 3][rx], PV[ry - 3][rx]),
+                                      make_float2(PU[ry - 2][rx], PV[ry - 2][rx]),
+                                      make_float2(PU[ry - 1][rx], PV[ry - 1][rx]), make_float2(PU[ry][rx], PV[ry][rx]),
+                                      make_float2(PU[ry + 1][rx], PV[ry + 1][rx]),
+                                      make_float2(PU[ry + 2][rx], PV[ry + 2][rx]), f2(eps));
     } else if (ty == 2) {  // north y faces of w, column tx
       const int ry = ZY + ZHY, rx = tx + ZHX;
       float f = 0.f;
       if (k >= 1 && k < nz)
-        f = weno_flux(0.5f * (rm * eprev + r * PV[ry][rx]), PW[ry - 3][rx], PW[ry - 2][rx], PW[ry - 1][rx],
+        f = weno_flux(V16 ? 0.5f * (rm * eprev + r * PV[ry][rx]) : mean(rm, eprev, r, PV[ry][rx]),
+                      PW[ry - 3][rx], PW[ry - 2][rx], PW[ry - 1][rx],
                       PW[ry][rx], PW[ry + 1][rx], PW[ry + 2][rx], eps);
       yW[ZY][tx] = f;
       eprev = PV[ry][rx];
@@ -617,14 +673,21 @@ __global__ void __launch_bounds__(ZNT, 3) k_weno_momentum_zm(Dims d, Phys ph, Co
       const int ry = tx + ZHY, rx = ZX + ZHX;
       float f = 0.f;
       if (k >= 1 && k < nz)
-        f = weno_flux(0.5f * (rm * eprev + r * PU[ry][rx]), PW[ry][rx - 3], PW[ry][rx - 2], PW[ry][rx - 1],
+        f = weno_flux(V16 ? 0.5f * (rm * eprev + r * PU[ry][rx]) : mean(rm, eprev, r, PU[ry][rx]),
+                      PW[ry][rx - 3], PW[ry][rx - 2], PW[ry][rx - 1],
                       PW[ry][rx], PW[ry][rx + 1], PW[ry][rx + 2], eps);
       xW[tx][ZX] = f;
       eprev = PU[ry][rx];
     }
     __syncthreads();
-    inUV = fma2(sub2(yUV[ty + 1][tx], yUV[ty][tx]), f2(-ph.rdy), mul2(sub2(xUV[ty][tx + 1], xUV[ty][tx]), f2(-ph.rdx)));
-    inW = fmaf(yW[ty + 1][tx] - yW[ty][tx], -ph.rdy, (xW[ty][tx + 1] - xW[ty][tx]) * -ph.rdx);
+    if (V16) {
+      inUV = fma2(sub2(yUV[ty + 1][tx], yUV[ty][tx]), f2(-ph.rdy), mul2(sub2(xUV[ty][tx + 1], xUV[ty][tx]), f2(-ph.rdx)));
+      inW = fmaf(yW[ty + 1][tx] - yW[ty][tx], -ph.rdy, (xW[ty][tx + 1] - xW[ty][tx]) * -ph.rdx);
+    } else {
+      const float2 xd = sub2(xUV[ty][tx + 1], xUV[ty][tx]), yd = sub2(yUV[ty + 1][tx], yUV[ty][tx]);
+      inUV = make_float2(sum2(xd.x, ph.rdx, yd.x, ph.rdy), sum2(xd.y, ph.rdx, yd.y, ph.rdy));
+      inW = sum2(xW[ty][tx + 1] - xW[ty][tx], ph.rdx, yW[ty + 1][tx] - yW[ty][tx], ph.rdy);
+    }
     corU = corUN;
     corV = corVN;
     dzC = dcC;

@@ -107,12 +107,15 @@ __device__ __forceinline__ float div_approx(float x, float y) {
   return r;
 }
 
+// B2: which of the two products of the middle smoothness keeps its rounding (the first where it says so)
+template <bool B2 = false>
 __device__ __forceinline__ float weno5(float a, float b, float c, float d, float e, float eps) {
   const float t1 = a - 2.f * b + c, t2 = a - 4.f * b + 3.f * c;
   const float t3 = b - 2.f * c + d, t4 = b - d;
   const float t5 = c - 2.f * d + e, t6 = 3.f * c - 4.f * d + e;
   const float b1 = (13.f / 12.f) * t1 * t1 + 0.25f * t2 * t2;
-  const float b2 = (13.f / 12.f) * t3 * t3 + 0.25f * t4 * t4;
+  const float b2 = B2 ? __fmaf_rn(0.25f * t4, t4, __fmul_rn((13.f / 12.f) * t3, t3))
+                      : (13.f / 12.f) * t3 * t3 + 0.25f * t4 * t4;
   const float b3 = (13.f / 12.f) * t5 * t5 + 0.25f * t6 * t6;
   const float tau = fabsf(b1 - b3);
   const float r1 = fminf(kRatioCap, div_approx(tau, b1 + eps));

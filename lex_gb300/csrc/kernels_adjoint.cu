@@ -619,11 +619,11 @@ __global__ void __launch_bounds__(ROW_T) k_adv_row_vjp(Dims d, Phys ph, Cols c, 
     if (cell && (f != 2 || k >= 1)) {
       float m = rk * u0;
       if (f == 0)
-        m = 0.5f * (LD(u, im) + u0) * rk;
+        m = mass_flux(LD(u, im), u0, rk);
       else if (f == 1)
-        m = 0.5f * (rk * LD(u, k * plane + wrapx(j - 1, ny) * nx + i) + m);
+        m = mass_flux(rk, LD(u, k * plane + wrapx(j - 1, ny) * nx + i), rk, u0);
       else if (f == 2)
-        m = 0.5f * (c.rho[k - 1] * LD(u, id - plane) + m);
+        m = mass_flux(c.rho[k - 1], LD(u, id - plane), rk, u0);
       const float Fb = (LD(a.cb[f], id) - LD(a.cb[f], im)) * ph.rdx;
       float s[6], g[6];
 #pragma unroll
@@ -670,15 +670,10 @@ __global__ void __launch_bounds__(MARCH_T) k_adv_march_vjp(Dims d, Phys ph, Cols
   // rows -5 .. ny + 4 of at least four
   auto at = [&](int p) { return base + (D == 1 ? wrapx(wrapx(p, ny), ny) : p) * stride; };
   auto inside = [&](int p) { return D == 1 || (p >= 0 && p < n); };
-  // the two winds of a face's mass flux (the same one for theta and qv) and their factors
+  // the two winds of a face's mass flux (theta and qv: one)
   const int da = f == 0 ? wrapx(i - 1, nx) - i : D == 2 && f == 1 ? (wrapx(r - 1, ny) - r) * nx : D == 1 && f == 2 ? -plane : 0;
   const int ha = f == D ? 1 : 0;   // the wind's own field: the points on either side of the face
-  const float half = f < 3 ? 0.5f : 0.f;
-  float w1 = f < 3 ? 0.5f : 1.f, w0 = half;
-  if (D == 1) {
-    w0 *= f == 2 ? c.rho[r - 1] : c.rho[r];
-    w1 *= c.rho[r];
-  }
+  const float ra = D == 1 ? (f == 2 ? c.rho[r - 1] : c.rho[r]) : 0.f, rb = D == 1 ? c.rho[r] : 0.f;
   // faces p0 - 2 .. p1 + 2 touch the chunk's points
   float s[6], acc[6];
 #pragma unroll
@@ -705,13 +700,8 @@ __global__ void __launch_bounds__(MARCH_T) k_adv_march_vjp(Dims d, Phys ph, Cols
     const float cbp = ncb, wa = nwa, wp = nw, o = nout;
     if (H < p1 + 2) load(H + 1);
     if (D == 1 || (H >= 1 && H < n)) {
-      float m;
-      if (D == 1)
-        m = w0 * wa + w1 * wp;
-      else if (f == 2)
-        m = 0.5f * (wa + wp) * c.rho[H - 1];
-      else
-        m = (w0 * wa + w1 * wp) * c.rho_face[H];
+      const float rc = D == 1 ? rb : f == 2 ? c.rho[H - 1] : c.rho_face[H];
+      const float m = f == D ? mass_flux(wa, wp, rc) : f > 2 ? rc * wp : mass_flux(D == 1 ? ra : rc, wa, rc, wp);
       const float Fb = (cbp - cbm) * rd;
       float g[6];
       const float W = D == 1 ? lateral_grad(m, s, eps, g) : vertical_grad(m, s, H, n, eps, g);

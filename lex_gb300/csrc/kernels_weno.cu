@@ -115,7 +115,7 @@ __device__ __forceinline__ float2 vflux6x2(float m, float2 sm3, float2 sm2, floa
 // 36.9 us (u, v, w); one 32 x 4 x 4 box with a 3-D halo per block took 27.2 (with a kernel of its own
 // for the divergence) and 37.5.  On such rows (V16 false) the marches keep the boxes' arithmetic, bit
 // for bit: divisions by rho0, u, v and w reconstructed one by one, products and sums contracted as diff,
-// mean, sum2 and sum3 say.  In the other rows' arithmetic (reciprocals, packed reconstructions) u, v and w
+// sum2 and sum3 say.  In the other rows' arithmetic (reciprocals, packed reconstructions) u, v and w
 // took 31.8 us, and the states differed in their last bits: that much moves the sign of a mass flux
 // somewhere, where an adjoint jumps (up to 3e-3 of its rms at single points).
 // ================================================================================================
@@ -205,11 +205,8 @@ struct ZLevel {
 };
 
 // Products and sums of the marches on rows of other lengths than multiples of 4, each rounded as written.
-// r a - s b, 0.5 (r a + s b) and a da + b db + c dc:
+// r a - s b and a da + b db + c dc:
 __device__ __forceinline__ float diff(float r, float a, float s, float b) { return __fmaf_rn(r, a, -__fmul_rn(s, b)); }
-__device__ __forceinline__ float mean(float r, float a, float s, float b) {
-  return 0.5f * __fmaf_rn(r, a, __fmul_rn(s, b));
-}
 __device__ __forceinline__ float sum2(float a, float da, float b, float db) { return __fmaf_rn(a, da, __fmul_rn(b, db)); }
 __device__ __forceinline__ float sum3(float a, float da, float b, float db, float c, float dc) {
   return __fmaf_rn(c, dc, sum2(a, da, b, db));
@@ -529,13 +526,12 @@ __global__ void __launch_bounds__(ZNT, 3) k_weno_momentum_zm(Dims d, Phys ph, Co
     float2 zUV = f2(0.f);
     if (k >= 1 && k < nz) {
       const float rf = c.rho_face[k];
-      const float2 m = V16 ? make_float2(0.5f * (rf * PW[ly][lx - 1] + rf * PW[ly][lx]),
-                                         0.5f * (rf * PW[ly - 1][lx] + rf * PW[ly][lx]))
-                           : make_float2(mean(rf, PW[ly][lx - 1], rf, PW[ly][lx]), mean(rf, PW[ly - 1][lx], rf, PW[ly][lx]));
+      const float2 m = make_float2(mass_flux(rf, PW[ly][lx - 1], rf, PW[ly][lx]),
+                                   mass_flux(rf, PW[ly - 1][lx], rf, PW[ly][lx]));
       zUV = vflux6_2m<V16>(m, make_float2(su[0], sv[0]), make_float2(su[1], sv[1]), make_float2(su[2], sv[2]),
                            make_float2(su[3], sv[3]), make_float2(su[4], sv[4]), make_float2(su[5], sv[5]), k, nz, eps);
     }
-    const float zW = (k >= 1) ? vflux6(0.5f * (sw[2] + sw[3]) * c.rho[k - 1], sw[0], sw[1], sw[2], sw[3], sw[4],
+    const float zW = (k >= 1) ? vflux6(mass_flux(sw[2], sw[3], c.rho[k - 1]), sw[0], sw[1], sw[2], sw[3], sw[4],
                                        sw[5], k, nz + 1, eps)
                               : 0.f;
     if (k > kb && col_own) {  // level k-1 complete
@@ -594,17 +590,15 @@ __global__ void __launch_bounds__(ZNT, 3) k_weno_momentum_zm(Dims d, Phys ph, Co
     const float r = c.rho[k], rm = k >= 1 ? c.rho[k - 1] : 0.f;
     auto xs = [&](const float(&P)[ZPY][ZPX], int ry, int rx, int o) { return P[ry][rx + o]; };
     {
-      const float2 mu = make_float2(0.5f * (PU[ly][lx - 1] + PU[ly][lx]) * r,          // cell between u's
-                                    V16 ? 0.5f * (r * PV[ly][lx - 1] + r * PV[ly][lx])     // corner
-                                        : mean(r, PV[ly][lx - 1], r, PV[ly][lx]));
+      const float2 mu = make_float2(mass_flux(PU[ly][lx - 1], PU[ly][lx], r),          // cell between u's
+                                    mass_flux(r, PV[ly][lx - 1], r, PV[ly][lx]));      // corner
       const float2 fu = weno_flux_2m<V16>(mu, make_float2(PU[ly][lx - 3], PU[ly - 3][lx]),
                                           make_float2(PU[ly][lx - 2], PU[ly - 2][lx]),
                                           make_float2(PU[ly][lx - 1], PU[ly - 1][lx]), make_float2(PU[ly][lx], PU[ly][lx]),
                                           make_float2(PU[ly][lx + 1], PU[ly + 1][lx]),
                                           make_float2(PU[ly][lx + 2], PU[ly + 2][lx]), f2(eps));
-      const float2 mv = make_float2(V16 ? 0.5f * (r * PU[ly - 1][lx] + r * PU[ly][lx])      // corner
-                                        : mean(r, PU[ly - 1][lx], r, PU[ly][lx]),
-                                    0.5f * (PV[ly - 1][lx] + PV[ly][lx]) * r);         // cell between v's
+      const float2 mv = make_float2(mass_flux(r, PU[ly - 1][lx], r, PU[ly][lx]),       // corner
+                                    mass_flux(PV[ly - 1][lx], PV[ly][lx], r));         // cell between v's
       const float2 fv = weno_flux_2m<V16>(mv, make_float2(PV[ly][lx - 3], PV[ly - 3][lx]),
                                           make_float2(PV[ly][lx - 2], PV[ly - 2][lx]),
                                           make_float2(PV[ly][lx - 1], PV[ly - 1][lx]), make_float2(PV[ly][lx], PV[ly][lx]),
@@ -614,8 +608,7 @@ __global__ void __launch_bounds__(ZNT, 3) k_weno_momentum_zm(Dims d, Phys ph, Co
       yUV[ty][tx] = make_float2(fu.y, fv.y);
     }
     if (k >= 1 && k < nz) {  // w's lateral faces on interior face levels
-      const float2 mw = V16 ? make_float2(0.5f * (rm * su[2] + r * su[3]), 0.5f * (rm * sv[2] + r * sv[3]))
-                            : make_float2(mean(rm, su[2], r, su[3]), mean(rm, sv[2], r, sv[3]));
+      const float2 mw = make_float2(mass_flux(rm, su[2], r, su[3]), mass_flux(rm, sv[2], r, sv[3]));
       const float2 fw = weno_flux_2m<V16>(mw, make_float2(PW[ly][lx - 3], PW[ly - 3][lx]),
                                           make_float2(PW[ly][lx - 2], PW[ly - 2][lx]),
                                           make_float2(PW[ly][lx - 1], PW[ly - 1][lx]), make_float2(PW[ly][lx], PW[ly][lx]),
@@ -641,9 +634,8 @@ __global__ void __launch_bounds__(ZNT, 3) k_weno_momentum_zm(Dims d, Phys ph, Co
     }
     if (ty == 0 && tx < ZY) {  // east x faces of u and v, row tx
       const int ry = tx + ZHY, rx = ZX + ZHX;
-      const float2 m = make_float2(0.5f * (PU[ry][rx - 1] + PU[ry][rx]) * r,
-                                   V16 ? 0.5f * (r * PU[ry - 1][rx] + r * PU[ry][rx])
-                                       : mean(r, PU[ry - 1][rx], r, PU[ry][rx]));
+      const float2 m = make_float2(mass_flux(PU[ry][rx - 1], PU[ry][rx], r),
+                                   mass_flux(r, PU[ry - 1][rx], r, PU[ry][rx]));
       xUV[tx][ZX] = weno_flux_2m<V16>(m, make_float2(xs(PU, ry, rx, -3), xs(PV, ry, rx, -3)),
                                       make_float2(xs(PU, ry, rx, -2), xs(PV, ry, rx, -2)),
                                       make_float2(xs(PU, ry, rx, -1), xs(PV, ry, rx, -1)),
@@ -652,9 +644,8 @@ __global__ void __launch_bounds__(ZNT, 3) k_weno_momentum_zm(Dims d, Phys ph, Co
                                       make_float2(xs(PU, ry, rx, 2), xs(PV, ry, rx, 2)), f2(eps));
     } else if (ty == 1) {  // north y faces of u and v, column tx
       const int ry = ZY + ZHY, rx = tx + ZHX;
-      const float2 m = make_float2(V16 ? 0.5f * (r * PV[ry][rx - 1] + r * PV[ry][rx])
-                                       : mean(r, PV[ry][rx - 1], r, PV[ry][rx]),
-                                   0.5f * (PV[ry - 1][rx] + PV[ry][rx]) * r);
+      const float2 m = make_float2(mass_flux(r, PV[ry][rx - 1], r, PV[ry][rx]),
+                                   mass_flux(PV[ry - 1][rx], PV[ry][rx], r));
       yUV[ZY][tx] = weno_flux_2m<V16>(m, make_float2(PU[ry - 3][rx], PV[ry - 3][rx]),
                                       make_float2(PU[ry - 2][rx], PV[ry - 2][rx]),
                                       make_float2(PU[ry - 1][rx], PV[ry - 1][rx]), make_float2(PU[ry][rx], PV[ry][rx]),
@@ -664,7 +655,7 @@ __global__ void __launch_bounds__(ZNT, 3) k_weno_momentum_zm(Dims d, Phys ph, Co
       const int ry = ZY + ZHY, rx = tx + ZHX;
       float f = 0.f;
       if (k >= 1 && k < nz)
-        f = weno_flux(V16 ? 0.5f * (rm * eprev + r * PV[ry][rx]) : mean(rm, eprev, r, PV[ry][rx]),
+        f = weno_flux(mass_flux(rm, eprev, r, PV[ry][rx]),
                       PW[ry - 3][rx], PW[ry - 2][rx], PW[ry - 1][rx],
                       PW[ry][rx], PW[ry + 1][rx], PW[ry + 2][rx], eps);
       yW[ZY][tx] = f;
@@ -673,7 +664,7 @@ __global__ void __launch_bounds__(ZNT, 3) k_weno_momentum_zm(Dims d, Phys ph, Co
       const int ry = tx + ZHY, rx = ZX + ZHX;
       float f = 0.f;
       if (k >= 1 && k < nz)
-        f = weno_flux(V16 ? 0.5f * (rm * eprev + r * PU[ry][rx]) : mean(rm, eprev, r, PU[ry][rx]),
+        f = weno_flux(mass_flux(rm, eprev, r, PU[ry][rx]),
                       PW[ry][rx - 3], PW[ry][rx - 2], PW[ry][rx - 1],
                       PW[ry][rx], PW[ry][rx + 1], PW[ry][rx + 2], eps);
       xW[tx][ZX] = f;

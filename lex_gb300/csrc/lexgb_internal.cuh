@@ -161,6 +161,18 @@ __device__ __forceinline__ float vrecon(const F& s, int f, int n, bool up, float
   }
 }
 
+// Mass flux through a face of u, v or w, whose sign picks the stencil: of the wind's own field, a cell of
+// density r between two of its faces; of another one, two faces with densities (or face densities) r and s.
+// The forward marches and the reverse pass take the sign from these and nothing else, each product and sum
+// rounded as written: where the two winds cancel, another contraction may give the other sign, and the
+// reverse pass would differentiate the stencil that the forward pass did not take.
+__device__ __forceinline__ float mass_flux(float a, float b, float r) {
+  return __fmul_rn(__fmul_rn(0.5f, __fadd_rn(a, b)), r);
+}
+__device__ __forceinline__ float mass_flux(float r, float a, float s, float b) {
+  return __fmul_rn(0.5f, __fmaf_rn(r, a, __fmul_rn(s, b)));
+}
+
 // jax.lax.select(m >= 0, m*pos, m*neg): ties take the positive branch.
 __device__ __forceinline__ float upwind(float m, float pos, float neg) { return m >= 0.f ? m * pos : m * neg; }
 

@@ -1078,8 +1078,9 @@ extern "C" int lexgb_cnn_net_forward(int nx, int ny, int nz, const float* x, con
     o.gelu = !last;
     o.creal = last ? NET_REAL : NET_COUT[l];
     o.compact = last;
-    // each layer stages its weights, which no kernel of this call writes, while the previous one drains
-    const cudaError_t e = conv3d(nx, ny, nz, NET_CIN[l], NET_COUT[l], act[l], w[l], o, st, true);
+    // each layer stages its weights, which no kernel of this call writes, while the previous one drains;
+    // not the first with x NULL: the kernel before it is the caller's, and may be the one that writes them
+    const cudaError_t e = conv3d(nx, ny, nz, NET_CIN[l], NET_COUT[l], act[l], w[l], o, st, l > 0 || x);
     if (e != cudaSuccess) return cnn_status(e, "lexgb_cnn_net_forward");
   }
   return LEXGB_OK;

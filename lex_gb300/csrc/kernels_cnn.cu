@@ -737,8 +737,9 @@ __global__ void k_sgs_pack(int nx, int ny, int nz, const PackIn in, uint4* __res
 // dl_models.py:172-182); w on the interior faces 1..nz-1 as the mean of the cells below and above
 // (bottom and lid untouched); each times the output range at its own point, rout[f][l][j][i]
 // (stride nz+1 levels: cells for theta and qv, west / south faces for u / v, faces 0..nz for w).
-// One thread per cell; it writes only its own cell and its own west, south and bottom faces.
-__global__ void k_sgs_unpack(int nx, int ny, int nz, const float* __restrict__ corr, const float* __restrict__ rout,
+// One thread per cell; it writes only its own cell and its own west, south and bottom faces.  corr is
+// still being written when the kernel's blocks start (no __restrict__: its loads stay behind pdl_wait).
+__global__ void k_sgs_unpack(int nx, int ny, int nz, const float* corr, const float* __restrict__ rout,
                              float* __restrict__ T, float* __restrict__ u, float* __restrict__ v, float* __restrict__ w,
                              float* __restrict__ q) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;

@@ -1261,32 +1261,45 @@ AdjWindows adj_windows(lexgb_ctx* c, AdjWork& w, int nstages) {
 // as one graph, launched on the bound stream.  A launch a kernel held small grids up: 64x64x64, two steps
 // and their reverse pass, 4.2 ms of which the GPU worked 2.9, as graphs 3.3 ms.  Not on the first runs, as
 // a constant that is learned changes the settings on every step, and the capture costs about as much as the
-// launches; not while the caller captures the bound stream.
+// launches; not while the caller captures the bound stream, on any run; and, until the settings change, not
+// after a graph could not be made.
 enum { ADJ_KEEP, ADJ_KEPT, ADJ_RECOMPUTED };
+constexpr int kNoGraph = -1;   // adj_runs: none could be made
+
+// the pass as a graph, captured on the context's own stream (the legacy default stream cannot be captured)
+extern "C++" template <class F>
+cudaGraphExec_t capture_adjoint(lexgb_ctx* c, const F& pass) {
+  cudaStream_t bound = c->stream;
+  cudaGraph_t g = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  c->stream = c->own_stream;
+  cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
+  if (e == cudaSuccess) {
+    const int st = pass();
+    e = cudaStreamEndCapture(c->stream, &g);
+    if (st == LEXGB_OK && e == cudaSuccess && cudaGraphInstantiate(&exec, g, 0) != cudaSuccess) exec = nullptr;
+    if (g) cudaGraphDestroy(g);
+  }
+  c->stream = bound;
+  if (!exec) cudaGetLastError();
+  return exec;
+}
+
 extern "C++" template <class F>
 int run_adjoint(lexgb_ctx* c, int which, const F& pass) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return pass();
+  }
+  if (cap != cudaStreamCaptureStatusNone) return pass();
   if (!c->adj_exec[which]) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess) {
-      cudaGetLastError();
+    if (c->adj_runs[which] == kNoGraph || ++c->adj_runs[which] < 3) return pass();
+    c->adj_exec[which] = capture_adjoint(c, pass);
+    if (!c->adj_exec[which]) {
+      c->adj_runs[which] = kNoGraph;
       return pass();
     }
-    if (cap != cudaStreamCaptureStatusNone || ++c->adj_runs[which] < 3) return pass();
-    cudaStream_t bound = c->stream;
-    c->stream = c->own_stream;   // as the step graph: the legacy default stream cannot be captured
-    cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) {
-      c->stream = bound;
-      return fail(LEXGB_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-    }
-    const int st = pass();
-    cudaGraph_t g = nullptr;
-    e = cudaStreamEndCapture(c->stream, &g);
-    c->stream = bound;
-    if (st == LEXGB_OK && e == cudaSuccess) e = cudaGraphInstantiate(&c->adj_exec[which], g, 0);
-    if (g) cudaGraphDestroy(g);
-    if (st != LEXGB_OK) return st;
-    if (e != cudaSuccess) return fail(LEXGB_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
   }
   CK(cudaGraphLaunch(c->adj_exec[which], c->stream));
   return LEXGB_OK;

@@ -52,3 +52,36 @@ def test_forward_reads_weights_that_the_kernel_before_it_wrote(built_lib, kernel
         lib.lexgb_cnn_set_kernel(0)
         k = ctypes.c_uint(0)
         assert lib.lexgb_cnn_take_timeouts(ctypes.byref(k)) == 0 and k.value == 0
+
+
+@pytest.mark.parametrize("rows,cols", [(0, 5), (7, 5), (0, 16), (7, 16), (0, 9), (3, 4)])
+def test_gradient_of_an_input_with_spare_rows_or_channels(built_lib, rows, cols):
+    """net_apply takes x with more rows than the grid has points and with padding channels: its gradient has
+    x's shape, zero where x takes no part, and none is returned where none is wanted."""
+    torch = pytest.importorskip("torch")
+    from lex_gb300 import sgs_cnn
+    dims = (16, 6, 5)
+    n = 16 * 6 * 5
+    net = sgs_cnn.SGSNet(seed=2, zero_last=False)
+    gen = torch.Generator(device="cpu").manual_seed(7)
+    x5 = torch.rand(n, 5, generator=gen).cuda().requires_grad_(True)
+    x5.data[:, cols:] = 0.0
+    gy = torch.randn(n, 5, generator=gen).cuda()
+    y = sgs_cnn.net_apply(net, x5, dims)
+    ref, = torch.autograd.grad(y, x5, gy)
+    x = torch.zeros(n + rows, cols, device="cuda")
+    k = min(cols, 5)
+    x[:n, :k] = x5.detach()[:, :k]
+    x.requires_grad_(True)
+    for t in net.params():
+        t.requires_grad_(True)
+    out = sgs_cnn.net_apply(net, x, dims)
+    assert torch.equal(out, y)
+    dx, dw = torch.autograd.grad(out, [x, net.w[0]], gy)
+    assert dx.shape == x.shape and dx.dtype == x.dtype
+    assert torch.equal(dx[:n, :k], ref[:, :k])
+    dx[:n, :k] = 0.0
+    assert not dx.any()
+    out = sgs_cnn.net_apply(net, x.detach(), dims)
+    only, = torch.autograd.grad(out, [net.w[0]], gy)
+    assert torch.allclose(only, dw, rtol=1e-4, atol=1e-5 * float(dw.abs().max()))

@@ -254,7 +254,8 @@ int lexgb_step_vjp_kept(lexgb_ctx *ctx, const float *const ybar[6], float *xbar[
  *   accumulation: y = act(conv(x, w) + bias); nx a multiple of 16, cin a multiple of 16 (padding
  *   channels of x zero), cout 8, 16 or 32; w [27][cout][cin] BF16 (offset (dz+1)*9+(dy+1)*3+(dx+1));
  *   optional outputs: pre (FP32 pre-activation), y_bf16, y_f32; gelu: tanh-GELU (flax nn.gelu);
- *   output channels >= creal are written as zero.  With the offsets mirrored and cin/cout swapped
+ *   output channels >= creal are written as zero; x and w 16-byte aligned for cin 16 or 32, outputs
+ *   4-byte (LEXGB_ERR_ARG else).  With the offsets mirrored and cin/cout swapped
  *   in w it is the gradient with respect to the input.
  * lexgb_cnn_gelu_bwd: g = dy * GELU'(pre) (pre NULL: g = dy), FP32 [npts][c] -> BF16 [npts][cpad].
  * lexgb_cnn_conv3d_dw: dw[27][cout][cin] += sum_p g[p][co] x[p+off][ci], db[cout] += sum_p g[p][co]
@@ -284,14 +285,14 @@ int lexgb_cnn_conv3d_dw(int nx, int ny, int nz, int cin, int cout, int gstride, 
                         float *dw, float *db, void *stream);
 /* One training pass of the network (5 -> 32 -> 32 -> 32 -> 5; npts = nx ny nz points, nx a multiple of
  * 16) in one call each way.  w: the layers' BF16 weights [27][cout][cin] with (cin, cout) = (16, 32),
- * (32, 32), (32, 32), (32, 8); b: FP32 biases.
+ * (32, 32), (32, 32), (32, 8); b: FP32 biases.  w, act and work are 16-byte aligned (LEXGB_ERR_ARG else).
  * lexgb_cnn_net_forward: x [npts][5] FP32 (NULL: act[0] holds the input already, [npts][16] BF16 with
  *   zero padding channels) -> out [npts][5] FP32; kept for the backward pass: act[0] [npts][16], act[1..3]
  *   [npts][32] BF16 (each layer's input) and pre[0..2] [npts][32] FP32 (pre-activations).
  * lexgb_cnn_net_backward: gout [npts][5] FP32 -> dx [npts][5] FP32 and grads (FP32, overwritten): dw of
- *   the four layers in w's layout, then db (32, 32, 32, 8).  work: (64 npts + 82944) BF16 of scratch,
- *   16-byte aligned.  Each layer's input gradient takes GELU' of the layer below and that layer's bias
- *   sums in the convolution's epilogue. */
+ *   the four layers in w's layout, then db (32, 32, 32, 8).  work: (64 npts + 82944) BF16 of scratch.
+ *   Each layer's input gradient takes GELU' of the layer below and that layer's bias sums in the
+ *   convolution's epilogue. */
 int lexgb_cnn_net_forward(int nx, int ny, int nz, const float *x, const void *const w[4], const float *const b[4],
                           void *const act[4], float *const pre[3], float *out, void *stream);
 int lexgb_cnn_net_backward(int nx, int ny, int nz, const float *gout, const void *const w[4],

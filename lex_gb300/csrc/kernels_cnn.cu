@@ -963,6 +963,7 @@ int cnn_status(cudaError_t e, const char* what) {
   lexgb::record_error(std::string(what) + ": " + cudaGetErrorString(e));
   return LEXGB_ERR_CUDA;
 }
+bool aligned(const void* p, uintptr_t to) { return (uintptr_t)p % to == 0; }
 int cnn_arg(const char* msg) {
   lexgb::record_error(msg);
   return LEXGB_ERR_ARG;
@@ -977,6 +978,11 @@ extern "C" int lexgb_cnn_conv3d(int nx, int ny, int nz, int cin, int cout, const
   if (cin <= 0 || cin % 16) return cnn_arg("lexgb_cnn_conv3d: cin must be a positive multiple of 16");
   if (!(cout == 8 || cout == 16 || cout == 32)) return cnn_arg("lexgb_cnn_conv3d: cout must be 8, 16 or 32");
   if (!x || !w || (!y_bf16 && !y_f32 && !pre)) return cnn_arg("lexgb_cnn_conv3d: null argument");
+  // x and w are read, and y_bf16 is stored, in pieces of 16 and 4 bytes (4 and 2 for more input channels)
+  const bool wide = cin == 16 || cin == 32;
+  if (!aligned(x, wide ? 16 : 4) || !aligned(w, wide ? 16 : 4) || !aligned(y_bf16, wide ? 4 : 2) ||
+      !aligned(bias, 4) || !aligned(pre, 4) || !aligned(y_f32, 4))
+    return cnn_arg("lexgb_cnn_conv3d: x and w must be 16-byte aligned (cin 16 or 32), bias and outputs 4-byte");
   const long long warps = (long long)(nx / 16) * ny * nz;
   const unsigned blocks = (unsigned)((warps + 3) / 4);
   cudaStream_t st = (cudaStream_t)stream;
@@ -1047,10 +1053,13 @@ unsigned pad_blocks(long long n) {
   const long long b = (n + 255) / 256;
   return (unsigned)(b < 1216 ? b : 1216);   // 8 blocks per SM: few additions to db
 }
-bool net_args(int nx, int ny, int nz, const void* const* p, int np) {
+// the grid; n16 pointers that move in 16-byte pieces (16-byte aligned), and n4 of floats
+bool net_args(int nx, int ny, int nz, const void* const* p16, int n16, const void* const* p4, int n4) {
   if (nx <= 0 || ny <= 0 || nz <= 0 || nx % 16) return false;
-  for (int i = 0; i < np; ++i)
-    if (!p[i]) return false;
+  for (int i = 0; i < n16; ++i)
+    if (!p16[i] || !aligned(p16[i], 16)) return false;
+  for (int i = 0; i < n4; ++i)
+    if (!p4[i] || !aligned(p4[i], 4)) return false;
   return true;
 }
 }  // namespace
@@ -1060,9 +1069,10 @@ extern "C" int lexgb_cnn_net_forward(int nx, int ny, int nz, const float* x, con
                                      void* stream) {
   using namespace lexgb;
   if (!w || !b || !act || !pre || !out) return cnn_arg("lexgb_cnn_net_forward: null argument");
-  const void* all[15] = {w[0], w[1], w[2], w[3], b[0], b[1], b[2], b[3], act[0], act[1], act[2], act[3], pre[0], pre[1], pre[2]};
-  if (!net_args(nx, ny, nz, all, 15))
-    return cnn_arg("lexgb_cnn_net_forward: null argument, or nx not a positive multiple of 16");
+  const void* p16[8] = {w[0], w[1], w[2], w[3], act[0], act[1], act[2], act[3]};
+  const void* p4[9] = {b[0], b[1], b[2], b[3], pre[0], pre[1], pre[2], out, x ? x : out};
+  if (!net_args(nx, ny, nz, p16, 8, p4, 9))
+    return cnn_arg("lexgb_cnn_net_forward: null argument, nx not a positive multiple of 16, or w or act not 16-byte aligned");
   cudaStream_t st = (cudaStream_t)stream;
   const long long n = (long long)nx * ny * nz;
   if (x) {
@@ -1092,9 +1102,11 @@ extern "C" int lexgb_cnn_net_backward(int nx, int ny, int nz, const float* gout,
                                       float* dx, void* stream) {
   using namespace lexgb;
   if (!gout || !w || !act || !pre || !work || !grads || !dx) return cnn_arg("lexgb_cnn_net_backward: null argument");
-  const void* all[11] = {w[0], w[1], w[2], w[3], act[0], act[1], act[2], act[3], pre[0], pre[1], pre[2]};
-  if (!net_args(nx, ny, nz, all, 11))
-    return cnn_arg("lexgb_cnn_net_backward: null argument, or nx not a positive multiple of 16");
+  const void* p16[9] = {w[0], w[1], w[2], w[3], act[0], act[1], act[2], act[3], work};
+  const void* p4[6] = {pre[0], pre[1], pre[2], gout, grads, dx};
+  if (!net_args(nx, ny, nz, p16, 9, p4, 6))
+    return cnn_arg("lexgb_cnn_net_backward: null argument, nx not a positive multiple of 16, or w, act or work not "
+                   "16-byte aligned");
   cudaStream_t st = (cudaStream_t)stream;
   const long long n = (long long)nx * ny * nz;
   // work: two gradients of 32 channels (the first also holds the 16 channels at the output), then the

@@ -272,11 +272,10 @@ constexpr int SGS_CIN[4] = {16, 32, 32, 32}, SGS_COUT[4] = {32, 32, 32, 8};
 
 int run_sgs(lexgb_ctx* c) {
   const Dims& d = c->d;
-  // programmatic dependent launches only on a created stream (the step graph is captured on the
-  // context's own stream); on the legacy or per-thread default stream, plain stream order
-  const bool pdl = c->stream != nullptr && c->stream != cudaStreamLegacy && c->stream != cudaStreamPerThread;
-  // programmatic dependents: the weights and biases are the context's copies, written only by
-  // lexgb_set_sgs_net, so each layer stages them while the previous kernel finishes
+  // programmatic dependents, as the acoustic sub-steps on any stream: the weights and biases are the
+  // context's copies, written only by lexgb_set_sgs_net and at least one ordinary launch of the step ago, so
+  // each layer stages them while the previous kernel finishes
+  const bool pdl = true;
   CK(launch_sgs_input(d.nx, d.ny, d.nz, c->A.T, c->A.u, c->A.v, c->A.w, c->A.q, (float)c->theta_ref, c->sgs_lo,
                       c->sgs_rin, c->sgs_x, c->sgs_w[0], c->sgs_b[0], c->sgs_a0, c->stream, pdl));
   const void* in[4] = {c->sgs_x, c->sgs_a0, c->sgs_a1, c->sgs_a0};

@@ -62,3 +62,23 @@ def test_steps_have_the_same_bits_however_submitted(built_lib, dims):
                 assert all(torch.isfinite(a).all() for a in y)
             for a, b in zip(y, ref):
                 assert torch.equal(a, b), how
+
+
+def test_corrected_steps_have_the_same_bits_however_submitted(built_lib):
+    import torch
+    from lex_gb300 import sgs_cnn
+    dims = (32, 24, 32)
+    S, qv0 = solver(*dims)
+    with S:
+        x = state(*dims, qv0)
+        kelvin = (x[0] + 300.0,) + x[1:]
+        scale = sgs_cnn.make_scale([kelvin])
+        scale["rout"] = 0.01 * scale["rout"]
+        sgs_cnn.attach(S, sgs_cnn.SGSNet(seed=4, zero_last=False), scale)
+        ref = None
+        for how, y in runs(S, x):
+            if ref is None:
+                ref = y
+                assert all(torch.isfinite(a).all() for a in y)
+            for a, b in zip(y, ref):
+                assert torch.equal(a, b), how

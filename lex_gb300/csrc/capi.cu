@@ -394,8 +394,9 @@ extern "C" {
 // set-aside is a limit of this process's context; failures leave normal caching.
 //
 // Only where the four fields take at most half of the L2: the set-aside is lost to everything else.
-// Measured per big step with and without (us): 192x192x96 (57 MB) 2107 and 2185, 208x208x104 (73 MB)
-// 3062 and 3053, 224x224x112 (90 MB) 4132 and 3584, 240x240x120 (111 MB) 5512 and 4867.
+// Measured per big step without SGS, with and without, a process each (us): 192x192x96 (57 MB) 1932 and
+// 2011, 208x208x104 (73 MB) 2651 and 2648, 224x224x112 (90 MB) 3701 and 3169, 240x240x120 (111 MB) 4618 and
+// 3981.  A set-aside once raised stays for the process: 240x240x120 after a solver with 57 MB takes 4207.
 static bool l2_window_pays(int dev, size_t bytes) {
   int l2 = 0;
   return cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) == cudaSuccess && bytes <= (size_t)l2 / 2;

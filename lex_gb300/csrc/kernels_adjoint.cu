@@ -254,9 +254,11 @@ __device__ __forceinline__ AcCol acoustic_col(const Cols& c, int k, int nz) {
 // fields read, four written, five accumulated: 96 bytes a cell, 84 on average with the wind accumulators
 // updated every other sub-step, from the sub-step's result and from its input, which is the result of the
 // one before.  Bound by the memory's latency (162 registers, 12 warps an SM, DRAM at 41 %): 192x192x96
-// 95 us a sub-step when the accumulators were read after the stores, and so a second trip to memory, 81 us
-// with their lines on the way to L2 from the start.  Tried: the accumulators in registers from the start
-// (198 of them: 85 us), two cells a thread and twice the warps (86), programmatic dependent launch (no gain).
+// 66.3 us a sub-step (launch list; 109 when the kernel read the accumulators after the stores, in every
+// sub-step and through a persisting window of their own), 68.1 without their lines on the way to L2 from the
+// start, 72.6 with the winds' updated in every sub-step.  Slower, by 2 to 4 % of the pass: the accumulators in
+// registers from the start (198 of them), two cells a thread and twice the warps; programmatic dependent
+// launch gained nothing.
 template <int V>
 struct VecF;
 template <>

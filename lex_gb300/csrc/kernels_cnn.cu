@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(ConvSmem<CIN, COUT>::THREADS)
     k_conv3d_smem(int nx, int ny, int nz, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                   const ConvEpilogue o, int early_weights) {
   using L = ConvSmem<CIN, COUT>;
-  constexpr int CP = L::CP, NT = L::NT, KC = CIN / 16, CH = CIN / 8;  // CH: 16-byte chunks a row
+  constexpr int CP = L::CP, NT = L::NT, KC = CIN / 16;
   extern __shared__ __align__(16) __nv_bfloat16 conv_smem[];
   __nv_bfloat16* Ws = conv_smem;
   __nv_bfloat16* As = conv_smem + L::W_ELEMS;
@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(ConvSmem2<CIN, COUT>::THREADS)
                    const __nv_bfloat16* __restrict__ w, const ConvEpilogue o, int early_weights) {
   using L = ConvSmem2<CIN, COUT>;
   using S1 = ConvSmem<CIN, COUT>;
-  constexpr int CP = S1::CP, NT = S1::NT, KC = CIN / 16, CH = CIN / 8, PS = L::PS, PB = CONV_TY * 16 * PS;
+  constexpr int CP = S1::CP, NT = S1::NT, KC = CIN / 16, PS = L::PS, PB = CONV_TY * 16 * PS;
   extern __shared__ __align__(16) __nv_bfloat16 conv_smem[];
   __nv_bfloat16* Ws = conv_smem;
   __nv_bfloat16* As = conv_smem + S1::W_ELEMS;
@@ -1051,7 +1051,7 @@ constexpr int NET_REAL = 5;
 
 unsigned pad_blocks(long long n) {
   const long long b = (n + 255) / 256;
-  return (unsigned)(b < 1216 ? b : 1216);   // 8 blocks per SM: few additions to db
+  return (unsigned)(b < 1216 ? b : 1216);   // few additions to db: 8 blocks on each of 152 SMs
 }
 // the grid; n16 pointers that move in 16-byte pieces (16-byte aligned), and n4 of floats
 bool net_args(int nx, int ny, int nz, const void* const* p16, int n16, const void* const* p4, int n4) {

@@ -837,8 +837,8 @@ bool make_xmap(CUtensorMap* map, const void* x, int nx, int ny, int nz, int cin)
 // epilogue), an SM holds two blocks and takes their planes one after another; a lone block leaves
 // gaps, about 1.6 times the time, and with 55 KB of weights a block (wbytes) more where blocks on most
 // SMs fetch them at once.  (32 -> 32 channels, us: 128x128x64 with 5 levels 125, 10: 103, 32, which this
-// picks: 96; 64^3 4: 43, 8, picked: 36, 16: 43; 64x64x32 4, picked: 25, 8: 27; a corrected step at
-// 32^3 with 2 levels 154.4, 3, picked: 151.9, 4: 155.3.)
+// picks: 96; 64^3 4: 43, 8, picked: 36, 16: 43; 64x64x32 4, picked: 25, 8: 27; with this kernel forced, a
+// corrected step at 32^3 with 2 levels 154.4, 3, picked: 151.9, 4: 155.3.)
 int tc_levels(int tiles, int nz, int sms, int wbytes) {
   int zc = nz;
   double best = -1.0;

@@ -11,8 +11,9 @@ struct AcousticVjpArgs {
   const float *un, *vn, *wn;             // output winds of the sub-step
   const float *unb, *vnb, *wnb, *pnb;    // adjoint of the output
   float *ub, *vb, *wb, *pb;              // adjoint of the input (written)
-  float *Rub, *Rvb, *Rwb, *trhob, *psb;  // accumulated
-  int acc;  // to Rub, Rvb, Rwb: 0 nothing, 1 ub, vb, wb, 2 those and unb, vnb, wnb
+  float *Rub, *Rvb, *Rwb;  // accumulated as `acc` says: 0 not, 1 dtau (ub, vb, wb), 2 those and dtau (unb, vnb, wnb)
+  float *trhob, *psb;      // accumulated
+  int acc;
 };
 
 // Pointwise part of one stage backwards (after its acoustic loop).
@@ -59,7 +60,6 @@ cudaError_t launch_sum_scaled(long long n, const float* x, double scale, double*
 cudaError_t launch_smag_vjp(const Dims&, const Phys&, const Cols&, State x0, const SmagLin&, const SmagVjpArgs&,
                             cudaStream_t);
 
-// win: an L2 access-policy window for the launch (the accumulators)
 cudaError_t launch_acoustic_vjp(const Dims&, const Phys&, const Cols&, const AcousticVjpArgs&, float dtau,
                                 cudaStream_t);
 cudaError_t launch_stage_pointwise_vjp(const Dims&, const Phys&, const Cols&, const StageVjpArgs&, cudaStream_t);

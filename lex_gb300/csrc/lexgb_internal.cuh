@@ -142,25 +142,6 @@ __device__ __forceinline__ float weno3(float a, float b, float c, float eps) {
   return div_approx(w1 * (-0.5f * a + 1.5f * b) + w2 * (0.5f * b + 0.5f * c), w1 + w2);
 }
 
-// Vertical face value between column entries f-1 and f of an n-entry column s(0..n-1),
-// for upward (m >= 0) or downward flow; zero at f = 0 and f = n.  Centred / WENO3 next to
-// the ends exactly as vertical_flux_scalar2 / _u2 / _v2 / _w2 do.
-template <class F>
-__device__ __forceinline__ float vrecon(const F& s, int f, int n, bool up, float eps) {
-  if (f <= 0 || f >= n) return 0.f;
-  if (up) {
-    if (f == 1) return 0.5f * (s(0) + s(1));
-    if (f == 2) return weno3(s(0), s(1), s(2), eps);
-    if (f == n - 1) return weno3(s(n - 3), s(n - 2), s(n - 1), eps);
-    return weno5(s(f - 3), s(f - 2), s(f - 1), s(f), s(f + 1), eps);
-  } else {
-    if (f == 1) return weno3(s(2), s(1), s(0), eps);
-    if (f == n - 1) return 0.5f * (s(n - 1) + s(n - 2));
-    if (f == n - 2) return weno3(s(n - 1), s(n - 2), s(n - 3), eps);
-    return weno5(s(f + 2), s(f + 1), s(f), s(f - 1), s(f - 2), eps);
-  }
-}
-
 // Mass flux through a face of u, v or w, whose sign picks the stencil: of the wind's own field, a cell of
 // density r between two of its faces; of another one, two faces with densities (or face densities) r and s.
 // The forward marches and the reverse pass take the sign from these and nothing else, each product and sum
@@ -173,12 +154,9 @@ __device__ __forceinline__ float mass_flux(float r, float a, float s, float b) {
   return __fmul_rn(0.5f, __fmaf_rn(r, a, __fmul_rn(s, b)));
 }
 
-// jax.lax.select(m >= 0, m*pos, m*neg): ties take the positive branch.
-__device__ __forceinline__ float upwind(float m, float pos, float neg) { return m >= 0.f ? m * pos : m * neg; }
-
 // m * (upwind WENO5 value) at the face between s[-1] and s[0], given s[-3..2]: the stencil is
-// selected by the sign of the mass flux first, so only one reconstruction is evaluated
-// (the reference evaluates both and selects, advection.py:505).
+// selected by the sign of the mass flux first, so only one reconstruction is evaluated (the reference
+// evaluates both and selects, advection.py:505; ties take the positive branch, as there).
 __device__ __forceinline__ float weno_flux(float m, float sm3, float sm2, float sm1, float s0, float sp1, float sp2,
                                            float eps) {
   const bool p = m >= 0.f;
@@ -244,17 +222,6 @@ __device__ __forceinline__ float2 weno_flux_x2(float m, float2 sm3, float2 sm2, 
   const bool p = m >= 0.f;
   return mul2(f2(m), weno5x2(sel2(p, sm3, sp2), sel2(p, sm2, sp1), sel2(p, sm1, s0), sel2(p, s0, sm1),
                              sel2(p, sp1, sm2), eps));
-}
-
-// m * (upwind vertical face value) at face f of an n-entry column (see vrecon); zero at the ends.
-template <class F>
-__device__ __forceinline__ float vflux(float m, const F& s, int f, int n, float eps) {
-  if (f <= 0 || f >= n) return 0.f;
-  const bool up = m >= 0.f;
-  if (f >= 3 && f <= n - 3)
-    return m * weno5(up ? s(f - 3) : s(f + 2), up ? s(f - 2) : s(f + 1), up ? s(f - 1) : s(f), up ? s(f) : s(f - 1),
-                     up ? s(f + 1) : s(f - 2), eps);
-  return m * vrecon(s, f, n, up, eps);
 }
 
 // ---------------------------------------------------------------------------------------------

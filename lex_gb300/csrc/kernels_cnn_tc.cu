@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(TcLayout<CIN, COUT>::THREADS, 2)
 // y offsets -1, 0, +1 (and spare shifts whose rows are dropped), and with the gradient planes below, at and
 // above the input plane side by side in B the three z offsets too.  A costs the same however wide N is (its
 // reads from shared memory, about 60 cycles an MMA): with one MMA for each (dz, dx) a level took 72 of
-// them, and 32 -> 32 channels on 128x128x64 127 us; with 24, 62 us.  Each of the nine (dx, dz) pairs has
+// them, and 32 -> 32 channels on 128x128x64 127 us; with 24, 66 us (62 in longer chains, launch_dw).  Each of the nine (dx, dz) pairs has
 // its own accumulator in tensor memory; a block keeps them over all the (tile, level chunk) items
 // it takes and adds them to dW once, at the end.  Both operands are MN-major (the channels are
 // the contiguous 16 bytes of a core matrix; its 8 rows are 8 consecutive points along x):

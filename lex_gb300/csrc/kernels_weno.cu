@@ -29,7 +29,8 @@ __device__ __forceinline__ int pmod(int i, int n) {
 
 // face value through column face H (between entries H-1 and H of an n-entry column), given
 // s(H-3..H+2); entries outside 0..n-1 are never used; zero on the end faces.  Near-boundary
-// rules of vertical_flux_scalar2 and friends (advection.py:327-406).
+// rules of vertical_flux_scalar2 and friends (advection.py:327-406).  B2: weno5's, on the upward face next to
+// the upper end (u and v on rows of other lengths than multiples of 4, as the boxes rounded it).
 template <bool B2 = false>
 __device__ __forceinline__ float vflux6(float m, float sm3, float sm2, float sm1, float s0, float sp1, float sp2, int H,
                                         int n, float eps) {

@@ -107,7 +107,7 @@ __device__ __forceinline__ float div_approx(float x, float y) {
   return r;
 }
 
-// B2: which of the two products of the middle smoothness keeps its rounding (the first where it says so)
+// B2: of the two products of the middle smoothness the first is rounded before they are added
 template <bool B2 = false>
 __device__ __forceinline__ float weno5(float a, float b, float c, float d, float e, float eps) {
   const float t1 = a - 2.f * b + c, t2 = a - 4.f * b + 3.f * c;

@@ -128,7 +128,8 @@ class _NetFn(torch.autograd.Function):
         out = torch.empty(n, COUT_REAL, device="cuda")
         _lib.check(_lib.load().lexgb_cnn_net_forward(nx, ny, nz, _p(xin), _ptrs(net.wbf), _ptrs(net.b), _ptrs(acts),
                                                      _ptrs(pres), _p(out), _stream()))
-        ctx.net, ctx.dims, ctx.acts, ctx.pres, ctx.xshape = net, dims, acts, pres, x.shape
+        ctx.net, ctx.dims, ctx.acts, ctx.pres = net, dims, acts, pres
+        ctx.spare = None if five and x.shape[0] == n else x.shape   # rows past the grid or padding channels
         return out
 
     @staticmethod
@@ -142,11 +143,9 @@ class _NetFn(torch.autograd.Function):
         dx = torch.empty(n, CIN0, device="cuda")
         _lib.check(_lib.load().lexgb_cnn_net_backward(nx, ny, nz, _p(gout), _ptrs(net.wbf), _ptrs(ctx.acts),
                                                       _ptrs(ctx.pres), _p(work), _p(grads), _p(dx), _stream()))
-        if not ctx.needs_input_grad[0]:
-            dx = None
-        elif dx.shape != ctx.xshape:      # rows past the grid and padding channels take no part
-            full = torch.zeros(ctx.xshape, device="cuda")
-            full[:n, :CIN0] = dx[:, :ctx.xshape[1]]
+        if ctx.spare is not None:     # they take no part
+            full = torch.zeros(ctx.spare, device="cuda")
+            full[:n, :CIN0] = dx[:, :ctx.spare[1]]
             dx = full
         parts = torch.split(grads, WSIZES + nb)
         dw = tuple(g.view(27, cout, cin) for g, (cin, cout, _) in zip(parts, LAYERS))

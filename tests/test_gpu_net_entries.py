@@ -57,7 +57,7 @@ def test_forward_reads_weights_that_the_kernel_before_it_wrote(built_lib, kernel
 @pytest.mark.parametrize("rows,cols", [(0, 5), (7, 5), (0, 16), (7, 16), (0, 9), (3, 4)])
 def test_gradient_of_an_input_with_spare_rows_or_channels(built_lib, rows, cols):
     """net_apply takes x with more rows than the grid has points and with padding channels: its gradient has
-    x's shape, zero where x takes no part, and none is returned where none is wanted."""
+    x's shape, zero where x takes no part; without it the weights' gradients are the same."""
     torch = pytest.importorskip("torch")
     from lex_gb300 import sgs_cnn
     dims = (16, 6, 5)
